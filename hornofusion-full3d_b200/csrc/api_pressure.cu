@@ -29,18 +29,17 @@ int enqueue_tdma(eaf_cg* h, const HaloInputs& in, double* phi, int n_sweep) {
     EAF_CUDA(cudaMalloc((void**)&h->tdma_fac,
                         sizeof(double) * eaf::tdma_factor_doubles(h->nr, h->nth, h->nz)));
   }
-  h->last_grid = eaf::tdma_grid(h->nr, h->nth, h->nz);
-  h->last_block = 64;
+  eaf::tdma_launch_shape(h->nr, h->nth, h->nz, h->sms, &h->last_grid, &h->last_block);
   h->last_cluster = 1;
   EAF_CUDA(cudaEventRecord(h->ev[1], h->st));
   EAF_CUDA(cudaEventRecord(h->ev[2], h->st));
   if (n_sweep > 0) {
     EAF_CUDA(eaf::launch_tdma_f64(in, phi, h->nr, h->nth, h->nz, n_sweep, h->tdma_mbox,
-                                  h->tdma_fac, h->ws, h->timeout_ns, h->st));
+                                  h->tdma_fac, h->sms, h->ws, h->timeout_ns, h->st));
   }
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(cudaEventRecord(h->ev[4], h->st));
-  h->last_kernels = n_sweep > 0 ? 2 : 0;
+  h->last_kernels = n_sweep > 0 ? 3 + 3 * n_sweep : 0;
   return EAF_OK;
 }
 

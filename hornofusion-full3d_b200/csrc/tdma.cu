@@ -6,402 +6,725 @@
 // refreshing the theta halos before each direction. Each line solve reads
 // phi in place, so a line sees the NEW values of the lines solved before it
 // (Gauss-Seidel between lines) and the OLD values of the lines after it. The
-// kernel keeps exactly that: it is bit-identical to the sequential sweep.
+// kernels keep exactly that: the result is bit-identical to the sequential
+// sweep.
 //
-// Schedule. In a direction the lines form a grid (a, b) -- a the inner loop
-// index, b the outer -- and line (a, b) needs the new values of (a-1, b) and
-// (a, b-1) only. One warp owns one index of the grid and solves its chain of
-// lines in order: the in-chain dependency is the warp's own previous line,
-// kept in shared memory; the cross-chain one is the neighbouring owner's
-// line, which the owner also writes into a mailbox -- one slot per cell,
-// marked empty with a signalling NaN that arithmetic never produces -- and
-// the consumer polls the values themselves (bounded wait): one L2 round trip
-// per hand-over and no fence, since the data is the signal. The consumer
-// marks the slots empty again; slots alternate by sweep parity, and the
-// grid barrier between directions orders a reset before the slot's next
-// use. Owners are chosen so that the cross-chain value is the
-// THIRD term of the reference's right-hand side
-//   d = (Su + c1m*p1m) + c1p*p1p;  d = (d + c2m*p2m) + c2p*p2p
-// (p1m the in-chain neighbour, p2m the cross-chain one): everything before
-// it is summed while the warp waits. r lines: owner k, chain j; theta lines:
-// owner k, chain i; z lines: owner i, chain j. The critical path is about
-// (owners + chain) line solves plus one publish per owner.
+// Schedule. In a direction the lines form a grid (a, b) and line (a, b)
+// needs the new values of (a-1, b) and (a, b-1) only, so the critical path is
+// A + B - 1 dependent line solves. One warp (the solver of owner b) solves
+// its chain a = 0..A-1 in order, keeping its previous line in registers; the
+// line of the previous owner arrives through a hand-over slot whose value is
+// its own signal (slots hold a signalling NaN, which arithmetic never
+// produces, until written, and the consumer marks them empty again). G
+// adjacent owners share a block and hand over through shared memory; only
+// every G-th hand-over crosses blocks, through global memory (the mail warp
+// of the consuming block fetches it ahead of the solver). A loader warp per
+// solver copies the next lines' operands into a ring of buffers. The owner is
+// the shorter of the two line indices, never theta (its periodic halo must
+// keep the old values until its chain ends).
 //
-// Lane 0 runs the Thomas recurrences (two correctly rounded divisions per
-// cell, the reference's operation order); the other lanes gather and
-// scatter the line. Built with -fmad=false like the CG unit.
+// A line solve. Both halves of the Thomas solve that depend on phi,
+//   dp_i = (d_i - a_i dp_{i-1}) / m_i,   x_i = dp_i - cp_i x_{i+1},
+// are first-order recurrences of correctly rounded operations, sequential in
+// i. One lane running them took 95 ns an element, all of it latency. Here
+// each lane owns K = ceil(L/32) consecutive elements and needs only the
+// value entering its segment. A prefix scan of the segments' affine maps
+// gives that to a few ulps; then every lane runs its segment with the
+// sequential operations and hands its last value on, and the warp repeats
+// until no entering value changes by a single bit. Then, by induction from
+// lane 0, whose input is exact, every value is the sequential recurrence's,
+// whatever the scan delivered. Two passes are the rule, because a segment
+// contracts an error of a few ulps below a rounding; a line without
+// contraction takes up to 32, about the sequential cost. Per line of 120
+// elements the recurrences are 2 x 8 dependent elements long instead of
+// 2 x 120.
+//
+// What does not depend on phi -- the guarded pivots m_i, cp_i, y_i = 1/m_i
+// and the scan's segment products -- is computed once per call, by the same
+// fixed-point passes, in a record per line and direction that also holds the
+// line's coefficients in the order the solver's lanes read them, so a line
+// is one bulk copy plus the old neighbour values.
+// Built with -fmad=false like the CG unit.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "cg_common.cuh"
 #include "cg_kernels.h"
+#include "cluster_red.cuh"
 #include "recipdiv.cuh"
 #include "stencil.cuh"
+#include "stream_stage.cuh"
 #include "eafcg.h"
 
 namespace eaf {
 namespace {
 
-struct TdmaArgs {
-  HaloInputs in;  // aW..Su (phi unused: the kernel writes `phi`)
-  double* phi;
-  int nr, nth, nz;
-  long long sx, sxy;  // halo strides of j and k
-  int n_sweep;
-  int lmax;
-  double* mbox;       // hand-over slots, [2 parities][3 directions][n cells]
-  double* fac;        // line factors, [3 directions][m, y, cp][n cells]
-  GroupWs ws;
-  uint64_t timeout_ns;
-};
-
-// One direction's geometry: chain index a (stride sa), owner index b
-// (stride sb), line element e (stride se); cell (a, b, e) sits at halo
-// index base + a*sa + b*sb + e*se. c1m/c1p the coefficients of the first
-// neighbour pair of the right-hand side (stride s1; its minus side is the
-// chain's previous line), c2m/c2p the second pair (stride s2; its minus
-// side is the previous owner's line), lm/lp the in-line links.
-struct Dir {
-  int A, B, L;
-  long long sa, sb, se, s1, s2;
-  const double *c1m, *c1p, *c2m, *c2p, *lm, *lp;
-};
-
-__device__ __forceinline__ Dir make_dir(const TdmaArgs& a, int dir) {
-  Dir d;
-  const long long one = 1;
-  if (dir == 0) {  // r lines: element i, chain j, owner k
-    d.A = a.nth; d.B = a.nz; d.L = a.nr;
-    d.sa = a.sx; d.sb = a.sxy; d.se = one;
-    d.s1 = a.sx; d.c1m = a.in.aS; d.c1p = a.in.aN;
-    d.s2 = a.sxy; d.c2m = a.in.aB; d.c2p = a.in.aT;
-    d.lm = a.in.aW; d.lp = a.in.aE;
-  } else if (dir == 1) {  // theta lines: element j, chain i, owner k
-    d.A = a.nr; d.B = a.nz; d.L = a.nth;
-    d.sa = one; d.sb = a.sxy; d.se = a.sx;
-    d.s1 = one; d.c1m = a.in.aW; d.c1p = a.in.aE;
-    d.s2 = a.sxy; d.c2m = a.in.aB; d.c2p = a.in.aT;
-    d.lm = a.in.aS; d.lp = a.in.aN;
-  } else {  // z lines: element k, chain j, owner i
-    d.A = a.nth; d.B = a.nr; d.L = a.nz;
-    d.sa = a.sx; d.sb = one; d.se = a.sxy;
-    d.s1 = a.sx; d.c1m = a.in.aS; d.c1p = a.in.aN;
-    d.s2 = one; d.c2m = a.in.aW; d.c2p = a.in.aE;
-    d.lm = a.in.aB; d.lp = a.in.aT;
-  }
-  return d;
-}
-
 __device__ __forceinline__ double sign_small(double v) {
   return fabs(v) < kSmall ? copysign(kSmall, v) : v;
 }
 
-// Serial theta-periodic halo copy (src/mod_mpi_topology.f90:303-311) over
-// all (i, k) columns of the halo layout, each column's four copies in the
-// reference's statement order.
-__device__ void theta_wrap(const TdmaArgs& a) {
-  const long long ncol = (long long)(a.nr + 4) * (a.nz + 4);
-  for (long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
-       col += (long long)gridDim.x * blockDim.x) {
-    const long long i = col % (a.nr + 4), k = col / (a.nr + 4);
-    double* p = a.phi + i + a.sxy * k;  // (i-1, j = -1, k-1) at p[0]
-    auto J = [&](int j) { return (long long)(j + 1) * a.sx; };
-    // With nth == 1 the second and fourth statements read the columns the
-    // first and third just wrote; their values are taken from registers.
-    const double v0 = __ldcg(p + J(a.nth));
-    p[J(0)] = v0;
-    p[J(-1)] = a.nth == 1 ? v0 : __ldcg(p + J(a.nth - 1));
-    const double v1 = __ldcg(p + J(1));
-    p[J(a.nth + 1)] = v1;
-    p[J(a.nth + 2)] = a.nth == 1 ? v1 : __ldcg(p + J(2));
-  }
-}
+constexpr int kTdmaMaxLine = 1024;
+constexpr unsigned kAllLanes = 0xffffffffu;
 
-constexpr int kTdmaMaxLine = 1024;  // 32 elements per lane in a hand-over mask
+// Record of one line: nine arrays of W = 32 K doubles, element lane*K + k of
+// the line at [k][lane]; the scan's products, [step][lane], forward then
+// backward; four scalars.
+enum { kRSu, kR1m, kR1p, kR2m, kR2p, kRLo, kRM, kRY, kRCp, kRArrays };
+constexpr int kScanSteps = 5;
+enum { kRE0, kRE1, kRNf, kRNb, kRScalars };  // end links, scan steps needed
+
+// Sizes for K elements a lane: owners per block, operand buffers per owner
+// and hand-over slots per ring, as many as 220 KB of shared memory hold (at
+// least three buffers before a further owner).
+template <int K>
+struct LineGeo {
+  static constexpr int W = 32 * K;
+  static constexpr int kScanF = kRArrays * W;
+  static constexpr int kScanB = kScanF + 32 * kScanSteps;
+  static constexpr int kScalars = kScanB + 32 * kScanSteps;
+  static constexpr int kRec = kScalars + kRScalars;
+  static constexpr int kP1 = kRec, kP2 = kRec + W, kEnds = kRec + 2 * W;
+  static constexpr int kBuf = kEnds + 4;
+  static constexpr int kSlots = K <= 16 ? 4 : 2;
+  static constexpr int kLimit = 220 * 1024 / 8;
+  static constexpr int need(int g, int nb) { return g * (nb * kBuf + kSlots * W); }
+  static constexpr int owners() {
+    for (int g = 8; g > 1; --g)
+      if ((g <= 4 || K <= 2) && need(g, 3) <= kLimit) return g;
+    return 1;
+  }
+  static constexpr int G = owners();
+  static constexpr int NB = need(G, 4) <= kLimit ? 4 : need(G, 3) <= kLimit ? 3 : 2;
+  static constexpr int kThreads = 32 * (2 * G + 1);
+  static constexpr size_t kSmem = (size_t)need(G, NB) * sizeof(double);
+  static_assert(need(G, NB) <= kLimit, "line buffers exceed the shared memory");
+};
+
+// One direction. Cell (a, b, e) sits at halo index base + a*sa + b*sb + e*se;
+// pair 1 and pair 2 are the neighbour pairs of the right-hand side
+//   d = (Su + c1m*n1m) + c1p*n1p;  d = (d + c2m*n2m) + c2p*n2p
+// in the reference's order (strides s1, s2); the chain runs along pair 1
+// (chain1) or pair 2.
+struct Dir {
+  int A, B, L;
+  long long base, sa, sb, se, s1, s2;
+  const double *c1m, *c1p, *c2m, *c2p, *lm, *lp, *aP, *Su;
+  bool chain1;
+  bool b_fast;  // the owner index is the unit-stride one
+  int wrap;     // refresh theta halos: 0 no, 1 theta is the chain, 2 the line
+  long long sx;
+};
+
+struct FactorArgs {
+  Dir d;
+  double* rec;
+  double* mail;       // hand-over slots between blocks, marked empty here
+  double* phi;        // non-null: refresh the theta halos (first direction)
+  int nr, nth, nz;
+  int* err;
+};
+
+struct SweepArgs {
+  Dir d;
+  const double* rec;
+  double* mail;
+  double* phi;
+  int* err;
+  uint64_t timeout_ns;
+};
 
 // Empty hand-over slot: a signalling NaN (IEEE arithmetic only delivers
 // quiet NaNs, so no solution value has this pattern).
-#define kEmptySlot __longlong_as_double(0x7ff000017ff00001ll)
 constexpr unsigned long long kEmptyBits = 0x7ff000017ff00001ull;
+__device__ __forceinline__ double empty_slot() {
+  return __longlong_as_double((long long)kEmptyBits);
+}
+__device__ __forceinline__ bool is_empty(double v) {
+  return (unsigned long long)__double_as_longlong(v) == kEmptyBits;
+}
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
 
-// Line factors: the phi-independent half of `tdma` (src/mod_solver_3d.f90:
-// 30-38) -- the guarded pivots m_i = b_i - a_i cp_{i-1} (b_1 for i = 1) and
-// cp_i = c_i / m_i, in the reference's operations -- plus y_i = 1 / m_i, or
-// 0 where m_i is outside the safe range of div_by_recip. One thread per line
-// of every direction; the layout is [direction][m, y, cp][line][element].
-__global__ void tdma_factor_kernel(TdmaArgs a) {
-  const long long nA = (long long)a.nth * a.nz, nB = (long long)a.nr * a.nz,
-                  nC = (long long)a.nr * a.nth;
-  const long long n = (long long)a.nr * a.nth * a.nz;
-  const long long base = 2 + 2 * a.sx + 2 * a.sxy;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nA + nB + nC;
-       t += (long long)gridDim.x * blockDim.x) {
-    int dir;
-    long long line;
-    if (t < nA) { dir = 0; line = t; }
-    else if (t < nA + nB) { dir = 1; line = t - nA; }
-    else { dir = 2; line = t - nA - nB; }
-    const Dir d = make_dir(a, dir);
-    const int ch = (int)(line % d.A), b = (int)(line / d.A);
-    const long long q0 = base + ch * d.sa + b * d.sb;
-    double* M = a.fac + (long long)dir * 3 * n + line * d.L;
-    double* Y = M + n;
-    double* CP = Y + n;
-    double cp = 0.0;
-    for (int e = 0; e < d.L; ++e) {
+// Serial theta-periodic halo copy (src/mod_mpi_topology.f90:303-311) over
+// all (i, k) columns of the halo layout; with nth == 1 the second and fourth
+// statements read the columns that the first and third just wrote.
+__device__ void theta_wrap(double* phi, int nr, int nth, int nz) {
+  const long long sx = nr + 4, sxy = sx * (nth + 4);
+  const long long ncol = sx * (nz + 4);
+  for (long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x; col < ncol;
+       col += (long long)gridDim.x * blockDim.x) {
+    double* p = phi + col % sx + sxy * (col / sx);
+    auto J = [&](int j) { return (long long)(j + 1) * sx; };
+    const double v0 = p[J(nth)], v1 = p[J(1)];
+    const double vm = nth == 1 ? v0 : p[J(nth - 1)], v2 = nth == 1 ? v1 : p[J(2)];
+    p[J(0)] = v0;
+    p[J(-1)] = vm;
+    p[J(nth + 1)] = v1;
+    p[J(nth + 2)] = v2;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Line records: one warp per line. The pivots' recurrence (:30-38)
+//   m_i = guard(b_i - a_i cp_{i-1}),  cp_i = c_i / m_i
+// runs in the lanes' segments from the previous pass's entering values until
+// none changes (the first pass starts from zero: the recurrence forgets its
+// start within a few elements). Padding elements and the line's ends carry
+// values that leave the solver's recurrences untouched: lo = 0 in the first
+// element, cp = 0 in the last, and m = y = 1 with zero links beyond.
+// Bound by its stores: 60x120x84, 200 MB of records.
+// ---------------------------------------------------------------------------
+constexpr int kFactorBlock = 256;
+
+template <int K>
+__global__ void __launch_bounds__(kFactorBlock) tdma_factor_kernel(FactorArgs a) {
+  using Geo = LineGeo<K>;
+  const Dir& d = a.d;
+  const int lane = threadIdx.x & 31;
+  const long long lines = (long long)d.A * d.B;
+  const long long warps = (long long)gridDim.x * (kFactorBlock / 32);
+  if (a.phi) theta_wrap(a.phi, a.nr, a.nth, a.nz);
+  if (a.err && blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0;
+  for (long long t = (long long)blockIdx.x * (kFactorBlock / 32) + (threadIdx.x >> 5); t < lines;
+       t += warps) {
+    const int ch = d.b_fast ? (int)(t / d.B) : (int)(t % d.A);
+    const int b = d.b_fast ? (int)(t % d.B) : (int)(t / d.A);
+    const long long q0 = d.base + ch * d.sa + b * d.sb;
+    double* rec = a.rec + ((long long)b * d.A + ch) * Geo::kRec;
+    double lo[K], bb[K], cc[K], mm[K], cp[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
       const long long q = q0 + e * d.se;
-      const double ai = -d.lm[q], bi = a.in.aP[q], ci = -d.lp[q];
-      const double m = e == 0 ? sign_small(bi) : sign_small(bi - ai * cp);
-      cp = ci / m;
-      M[e] = m;
-      Y[e] = exp_in_safe_range(m) ? 1.0 / m : 0.0;
-      CP[e] = cp;
-      const long long slot = (long long)dir * n + line * d.L + e;
-      a.mbox[slot] = kEmptySlot;
-      a.mbox[3 * n + slot] = kEmptySlot;
+      const bool live = e < d.L;
+      lo[k] = live && e > 0 ? -d.lm[q] : 0.0;
+      bb[k] = live ? d.aP[q] : 1.0;
+      cc[k] = live ? -d.lp[q] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
+      const long long q = q0 + e * d.se;
+      const bool live = e < d.L;
+      const int o = k * 32 + lane;
+      rec[kRSu * Geo::W + o] = live ? d.Su[q] : 0.0;
+      rec[kR1m * Geo::W + o] = live ? d.c1m[q] : 0.0;
+      rec[kR1p * Geo::W + o] = live ? d.c1p[q] : 0.0;
+      rec[kR2m * Geo::W + o] = live ? d.c2m[q] : 0.0;
+      rec[kR2p * Geo::W + o] = live ? d.c2p[q] : 0.0;
+    }
+    double in = 0.0;
+    for (int pass = 0; pass <= 32; ++pass) {
+      double c = in;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        mm[k] = sign_small(bb[k] - lo[k] * c);
+        c = cc[k] / mm[k];
+        cp[k] = c;
+      }
+      double nin = __shfl_up_sync(kAllLanes, c, 1);
+      if (lane == 0) nin = 0.0;
+      if (__all_sync(kAllLanes, same_bits(nin, in))) break;
+      in = nin;
+    }
+    double pf = 1.0, pb = 1.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
+      const int o = k * 32 + lane;
+      const double y = exp_in_safe_range(mm[k]) ? 1.0 / mm[k] : 0.0;
+      const double cpe = e < d.L - 1 ? cp[k] : 0.0;
+      rec[kRLo * Geo::W + o] = lo[k];
+      rec[kRM * Geo::W + o] = mm[k];
+      rec[kRY * Geo::W + o] = y;
+      rec[kRCp * Geo::W + o] = cpe;
+      pf = pf * (-lo[k] * y);
+      pb = pb * -cpe;
+    }
+    // Scan products: step s adds the value 2^s lanes away times the product
+    // over the 2^s segments in between; a step whose products are all below
+    // 2^-56 (and those after it) would change nothing and is left out.
+    int nf = 0, nb = 0;
+#pragma unroll
+    for (int s = 0; s < kScanSteps; ++s) {
+      rec[Geo::kScanF + 32 * s + lane] = pf;
+      rec[Geo::kScanB + 32 * s + lane] = pb;
+      if (nf == s && __any_sync(kAllLanes, !(fabs(pf) < 0x1p-56))) nf = s + 1;
+      if (nb == s && __any_sync(kAllLanes, !(fabs(pb) < 0x1p-56))) nb = s + 1;
+      pf = pf * __shfl_up_sync(kAllLanes, pf, 1 << s);
+      pb = pb * __shfl_down_sync(kAllLanes, pb, 1 << s);
+    }
+    if (lane == 0) {
+      double* sc = rec + Geo::kScalars;
+      sc[kRE0] = d.lm[q0];
+      sc[kRE1] = d.lp[q0 + (long long)(d.L - 1) * d.se];
+      sc[kRNf] = (double)nf;
+      sc[kRNb] = (double)nb;
+    }
+    if (b % Geo::G == 0) {
+      double* slot = a.mail + ((long long)(b / Geo::G) * d.A + ch) * Geo::W;
+#pragma unroll
+      for (int k = 0; k < K; ++k) slot[k * 32 + lane] = empty_slot();
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Per owner, two warps: the LOADER fetches line ch+1 (coefficients, factors,
-// the old neighbour values it needs, the end couplings) into one of two
-// shared-memory buffers while the SOLVER finishes line ch; the solver then
-// only forms the right-hand side from shared memory plus the two new values
-// (its own previous line, the previous owner's mailbox) and runs the Thomas
-// recurrences. Hand-shake: named barriers FULL_k / EMPTY_k per buffer k (a
-// producer never arrives twice on one barrier before its consumer synced).
+// Sweep of one direction.
 // ---------------------------------------------------------------------------
-constexpr int kBarFull0 = 3, kBarEmpty0 = 5;  // FULL_k = 3 + k, EMPTY_k = 5 + k
-constexpr int kTdmaBlock = 64;
-constexpr int kBufArrays = 11;
-
-struct LineBuf {
-  double *su, *c1m, *c1t, *c2m, *c2t, *p1h, *p2h, *lo, *m, *y, *cp;
-};
-
-__device__ __forceinline__ LineBuf line_buf(double* base, int lmax) {
-  LineBuf b;
-  b.su = base;
-  b.c1m = b.su + lmax;
-  b.c1t = b.c1m + lmax;
-  b.c2m = b.c1t + lmax;
-  b.c2t = b.c2m + lmax;
-  b.p1h = b.c2t + lmax;
-  b.p2h = b.p1h + lmax;
-  b.lo = b.p2h + lmax;
-  b.m = b.lo + lmax;
-  b.y = b.m + lmax;
-  b.cp = b.y + lmax;
-  return b;
+__device__ __forceinline__ double ld_volatile_f64(const double* p) {
+  return *(const volatile double*)p;
+}
+__device__ __forceinline__ void st_volatile_f64(double* p, double v) {
+  *(volatile double*)p = v;
+}
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-// Loader: everything of line `ch` of owner `b` that does not depend on this
-// sweep's new values. Products are formed as the reference forms them
-// (c1p*p1p and c2p*p2p are added as whole terms); halo values for the
-// first line of the chain (p1) and for owner 0 (p2).
-__device__ __forceinline__ void load_line(const TdmaArgs& a, const Dir& d, const LineBuf& lb,
-                                          double* ends, long long q0, int ch, int b,
-                                          const double* fm, int lane) {
-  const double* __restrict__ phi = a.phi;
-  const double* __restrict__ Su = a.in.Su;
-  const long long n = (long long)a.nr * a.nth * a.nz;
-  for (int e = lane; e < d.L; e += 32) {
-    const long long q = q0 + e * d.se;
-    lb.su[e] = Su[q];
-    lb.c1m[e] = d.c1m[q];
-    lb.c1t[e] = d.c1p[q] * __ldcg(phi + q + d.s1);
-    lb.c2m[e] = d.c2m[q];
-    lb.c2t[e] = d.c2p[q] * __ldcg(phi + q + d.s2);
-    if (ch == 0) lb.p1h[e] = __ldcg(phi + q - d.s1);
-    if (b == 0) lb.p2h[e] = __ldcg(phi + q - d.s2);
-    lb.lo[e] = -d.lm[q];
-    lb.m[e] = __ldcg(fm + e);
-    lb.y[e] = __ldcg(fm + n + e);
-    lb.cp[e] = __ldcg(fm + 2 * n + e);
-  }
-  if (lane == 0) {
-    const long long qL = q0 + (long long)(d.L - 1) * d.se;
-    ends[0] = d.lm[q0] * __ldcg(phi + q0 - d.se);
-    ends[1] = d.lp[qL] * __ldcg(phi + qL + d.se);
-  }
-}
-
-// The phi-dependent half of tdma (src/mod_solver_3d.f90:32-45), lane 0:
-// dp_1 = d_1 / m_1, dp_i = (d_i - a_i dp_{i-1}) / m_i, x_i = dp_i - cp_i x_{i+1}.
-// The forward pass runs on the correction path only, its range conditions
-// OR-ed off the dependent chain; a line with any operand outside the safe
-// range (rare) is redone with `/` throughout. A zero numerator is exact on
-// this path as q = t*y itself (the correction would turn -0 into +0).
-__device__ __forceinline__ void thomas_line(const LineBuf& lb, const double* __restrict__ rhs,
-                                            double* __restrict__ dpa,
-                                            double* __restrict__ x, int L) {
-  const double* __restrict__ lo = lb.lo;
-  const double* __restrict__ mm = lb.m;
-  const double* __restrict__ yy = lb.y;
-  const double* __restrict__ cpa = lb.cp;
-  bool ok = yy[0] != 0.0 && (rhs[0] == 0.0 || exp_in_safe_range(rhs[0]));
-  double dp;
-  {
-    const double t = rhs[0], q = t * yy[0];
-    const double c = __fma_rn(__fma_rn(-q, mm[0], t), yy[0], q);
-    dp = t == 0.0 ? q : c;
-  }
-  dpa[0] = dp;
-  for (int i = 1; i < L; ++i) {
-    const double y = yy[i], m = mm[i];
-    const double t = rhs[i] - lo[i] * dp;
-    ok = ok & (y != 0.0) & (t == 0.0 || exp_in_safe_range(t));
-    const double q = t * y;
-    const double c = __fma_rn(__fma_rn(-q, m, t), y, q);
-    dp = t == 0.0 ? q : c;
-    dpa[i] = dp;
-  }
-  if (!ok) {
-    dp = rhs[0] / mm[0];
-    dpa[0] = dp;
-    for (int i = 1; i < L; ++i) {
-      dp = (rhs[i] - lo[i] * dp) / mm[i];
-      dpa[i] = dp;
-    }
-  }
-  double xv = dp;
-  x[L - 1] = xv;
-  for (int i = L - 2; i >= 0; --i) {
-    xv = dpa[i] - cpa[i] * xv;
-    x[i] = xv;
-  }
-}
-
-// Polls the previous owner's mailbox for line values (bounded); completes
-// rhs_e = (rhs_e + c2m_e * p2m_e) + c2t_e as they arrive and empties the
-// slots. False if the wait gave up.
-__device__ bool take_mailbox(const TdmaArgs& a, unsigned long long* slot, const LineBuf& lb,
-                             double* rhs, int L, int lane) {
-  unsigned pend = 0;
-  for (int k = 0; lane + 32 * k < L; ++k) pend |= 1u << k;
+// Bound of a polling loop; warp-uniform, true when the wait gives up (the
+// error word is set, by this wait's expiry or by another's).
+struct Patience {
   uint64_t t0 = 0;
   uint32_t spins = 0;
-  for (;;) {
-    for (int k = 0; lane + 32 * k < L; ++k) {
-      if (!(pend & (1u << k))) continue;
-      const int e = lane + 32 * k;
-      const unsigned long long v = ld_relaxed_u64(slot + e);
-      if (v == kEmptyBits) continue;
-      const double t = rhs[e] + lb.c2m[e] * __longlong_as_double((long long)v);
-      rhs[e] = t + lb.c2t[e];
-      slot[e] = kEmptyBits;
-      pend &= ~(1u << k);
-    }
-    if (!__any_sync(0xffffffffu, pend != 0)) return true;
-    if ((++spins & 63u) == 0) {
-      int stop = 0;
-      if (lane == 0) {
-        if (spins == 64u) t0 = global_ns();
-        if (ld_volatile_i32(a.ws.err) != 0) {
-          stop = 1;
-        } else if (global_ns() - t0 > a.timeout_ns) {
-          atomicCAS(a.ws.err, 0, (int)EAF_ETIMEOUT);
-          stop = 1;
-        }
+  __device__ __forceinline__ bool gives_up(int* err, uint64_t timeout_ns) {
+    if ((++spins & 63u) != 0) return false;
+    int stop = 0;
+    if ((threadIdx.x & 31) == 0) {
+      if (spins == 64u) t0 = global_ns();
+      if (ld_volatile_i32(err) != 0) {
+        stop = 1;
+      } else if (global_ns() - t0 > timeout_ns) {
+        atomicCAS(err, 0, (int)EAF_ETIMEOUT);
+        stop = 1;
       }
-      if (__shfl_sync(0xffffffffu, stop, 0)) return false;
+    }
+    return __shfl_sync(kAllLanes, stop, 0) != 0;
+  }
+};
+
+// Takes this lane's K values of a hand-over slot in shared memory once all
+// have arrived, and marks them empty; with `next`, also waits until the lane's
+// values of that slot (the one this line goes to) have been taken.
+template <int K>
+__device__ __forceinline__ bool take_slot(const SweepArgs& a, double* slot, const double* next,
+                                          int lane, double (&v)[K]) {
+  Patience w;
+  for (;;) {
+    bool ready = true;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      v[k] = ld_volatile_f64(slot + k * 32 + lane);
+      ready = ready && !is_empty(v[k]);
+    }
+    if (next) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) ready = ready && is_empty(ld_volatile_f64(next + k * 32 + lane));
+    }
+    if (__all_sync(kAllLanes, ready)) break;
+    if (w.gives_up(a.err, a.timeout_ns)) return false;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) st_volatile_f64(slot + k * 32 + lane, empty_slot());
+  return true;
+}
+
+// Writes a solved line from its buffer to phi, and the theta halos that it
+// completes: its own where the line is a theta column; where theta is the
+// chain, at the chain's end, the owner's columns (their old halo values are
+// no longer needed; the lane reads back values that it wrote).
+template <int K>
+__device__ __forceinline__ void write_line(const SweepArgs& a, const double* buf, int b, int ch,
+                                           int lane) {
+  using Geo = LineGeo<K>;
+  const Dir& d = a.d;
+  double* p = a.phi + d.base + ch * d.sa + b * d.sb;
+  double x[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) x[k] = buf[Geo::kP1 + k * 32 + lane];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int e = lane * K + k;
+    if (e < d.L) p[e * d.se] = x[k];
+  }
+  if (d.wrap == 2) {
+    const int n = d.L, n2 = n > 1 ? n - 2 : 0, one = n > 1 ? 1 : 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
+      if (e == n - 1) p[-d.se] = x[k];
+      if (e == n2) p[-2 * d.se] = x[k];
+      if (e == 0) p[n * d.se] = x[k];
+      if (e == one) p[(n + 1) * d.se] = x[k];
+    }
+  } else if (d.wrap == 1 && ch == d.A - 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
+      if (e >= d.L) continue;
+      double* c = a.phi + d.base + b * d.sb + e * d.se;  // (e, j = 1)
+      const int n = d.A;
+      const double v0 = x[k], v1 = c[0];
+      const double vm = n == 1 ? v0 : c[(n - 2) * d.sx], v2 = n == 1 ? v1 : c[d.sx];
+      c[-d.sx] = v0;
+      c[-2 * d.sx] = vm;
+      c[n * d.sx] = v1;
+      c[(n + 1) * d.sx] = v2;
     }
   }
 }
 
-__global__ void __launch_bounds__(kTdmaBlock) tdma_kernel(TdmaArgs a) {
-  extern __shared__ __align__(16) double sm[];
-  __shared__ double s_ends[2][2];
-  const LineBuf buf0 = line_buf(sm, a.lmax);
-  const LineBuf buf1 = line_buf(sm + kBufArrays * a.lmax, a.lmax);
-  double* s_x = sm + 2 * kBufArrays * a.lmax;
-  double* s_rhs = s_x + a.lmax;
-  double* s_dp = s_rhs + a.lmax;
-  const int lane = threadIdx.x & 31;
-  const bool loader = threadIdx.x >= 32;
-  Group g;
-  g.counter = a.ws.counter;
-  g.err = a.ws.err;
-  g.part = a.ws.part;
-  g.stage = nullptr;
-  g.nb = gridDim.x;
-  g.bid = blockIdx.x;
-  g.timeout_ns = a.timeout_ns;
-  g.epoch = 0;
-  const long long base = 2 + 2 * a.sx + 2 * a.sxy;  // cell (1, 1, 1)
-  double* __restrict__ phi = a.phi;
-  bool ok = true;
-  for (int sweep = 1; sweep <= a.n_sweep && ok; ++sweep) {
-    for (int dir = 0; dir < 3 && ok; ++dir) {
-      if (!(ok = group_barrier<1>(g))) break;
-      theta_wrap(a);
-      if (!(ok = group_barrier<1>(g))) break;
-      const Dir d = make_dir(a, dir);
-      const long long ncell = (long long)a.nr * a.nth * a.nz;
-      const double* fdir = a.fac + (long long)dir * 3 * ncell;
-      double* mb = a.mbox + ((long long)(sweep & 1) * 3 + dir) * ncell;
-      for (int b = blockIdx.x; b < d.B; b += gridDim.x) {
-        const long long qb = base + b * d.sb;
-        const long long lines_b = (long long)b * d.A * d.L;  // line (0, b)
-        if (loader) {
-          for (int ch = 0; ch < d.A; ++ch) {
-            const int k = ch & 1;
-            if (ch >= 2) named_sync(kBarEmpty0 + k, kTdmaBlock);
-            load_line(a, d, k ? buf1 : buf0, s_ends[k], qb + ch * d.sa, ch, b,
-                      fdir + lines_b + (long long)ch * d.L, lane);
-            named_arrive(kBarFull0 + k, kTdmaBlock);
-          }
-          continue;
-        }
-        double* mine = mb + lines_b;
-        unsigned long long* from =
-            b > 0 ? reinterpret_cast<unsigned long long*>(mb + lines_b - (long long)d.A * d.L)
-                  : nullptr;
-        const bool feeds = b + 1 < d.B;
-        bool live = true;  // false after a wait gave up: keep the hand-shake only
-        for (int ch = 0; ch < d.A; ++ch) {
-          const int k = ch & 1;
-          const LineBuf lb = k ? buf1 : buf0;
-          named_sync(kBarFull0 + k, kTdmaBlock);
-          if (live) {
-            const long long q0 = qb + ch * d.sa;
-            for (int e = lane; e < d.L; e += 32) {
-              const double p1m = ch == 0 ? lb.p1h[e] : s_x[e];
-              double t = lb.su[e] + lb.c1m[e] * p1m;
-              t = t + lb.c1t[e];
-              if (b == 0) {
-                t = t + lb.c2m[e] * lb.p2h[e];
-                t = t + lb.c2t[e];
-              }
-              s_rhs[e] = t;
-            }
-            if (b > 0 && !take_mailbox(a, from + (long long)ch * d.L, lb, s_rhs, d.L, lane))
-              live = false;
-            __syncwarp();
-            if (live) {
-              if (lane == 0) {
-                // lagged couplings of the segment ends (:299-302, :325-328, :352-355)
-                s_rhs[0] = s_rhs[0] + s_ends[k][0];
-                s_rhs[d.L - 1] = s_rhs[d.L - 1] + s_ends[k][1];
-                thomas_line(lb, s_rhs, s_dp, s_x, d.L);
-              }
-              __syncwarp();
-              for (int e = lane; e < d.L; e += 32) {
-                const double xv = s_x[e];
-                if (feeds) mine[(long long)ch * d.L + e] = xv;
-                phi[q0 + e * d.se] = xv;
-              }
-              __syncwarp();
-            }
-          }
-          if (ch + 2 < d.A) named_arrive(kBarEmpty0 + k, kTdmaBlock);
-        }
-      }
-      // A solver whose wait gave up kept the hand-shake and set the error
-      // word; the other waits see it and give up too, so every warp reaches
-      // the next group barrier and the launch ends with EAF_ETIMEOUT.
+// Position of a warp in its owners' lines, with the buffer it is in.
+template <int K>
+struct LineAt {
+  int b, ch = 0, st = 0;
+  uint32_t phase = 0;
+  __device__ explicit LineAt(int w) : b(blockIdx.x * LineGeo<K>::G + w) {}
+  __device__ __forceinline__ void next(int A) {
+    if (++st == LineGeo<K>::NB) {
+      st = 0;
+      phase ^= 1u;
     }
+    if (++ch == A) {
+      ch = 0;
+      b += gridDim.x * LineGeo<K>::G;
+    }
+  }
+};
+
+// Copies the operands of the owner's lines into its ring of buffers, as far
+// ahead as the solver has finished with them, and writes each finished line
+// out of its buffer before that is filled again. The old neighbour values may
+// be read at any time before the line is solved: a line's plus-side
+// neighbours are solved, and written, after it.
+template <int K>
+__device__ void load_lines(const SweepArgs& a, int w, double* bufs, uint64_t* full,
+                           uint64_t* empty, int lane) {
+  using Geo = LineGeo<K>;
+  const Dir& d = a.d;
+  LineAt<K> at(w), done(w);
+  int ahead = 0;  // lines issued and not yet written out
+  bool ok = true;
+  while (ok && done.b < d.B) {
+    if (ahead == Geo::NB || at.b >= d.B) {
+      ok = mbar_wait(&empty[done.st], done.phase, a.err, a.timeout_ns);
+      ok = __all_sync(kAllLanes, ok);
+      if (!ok) break;
+      write_line<K>(a, bufs + (size_t)done.st * Geo::kBuf, done.b, done.ch, lane);
+      done.next(d.A);
+      --ahead;
+    }
+    if (at.b >= d.B) continue;
+    double* buf = bufs + (size_t)at.st * Geo::kBuf;
+    const double* p = a.phi + d.base + at.ch * d.sa + at.b * d.sb;
+    if (lane == 0) {
+      mbar_arrive_expect(&full[at.st], Geo::kRec * 8);
+      bulk_copy_g2s(buf, a.rec + ((long long)at.b * d.A + at.ch) * Geo::kRec, Geo::kRec * 8,
+                    &full[at.st]);
+      cp_async8(buf + Geo::kEnds, p - d.se);
+      cp_async8(buf + Geo::kEnds + 1, p + d.L * d.se);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
+      if (e < d.L) {
+        cp_async8(buf + Geo::kP1 + k * 32 + lane, p + e * d.se + d.s1);
+        cp_async8(buf + Geo::kP2 + k * 32 + lane, p + e * d.se + d.s2);
+      }
+    }
+    cp_async_arrive(&full[at.st]);
+    at.next(d.A);
+    ++ahead;
+  }
+  // After a wait gave up: no copy may still be in flight into this block's
+  // memory when it leaves.
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  for (; ahead > 0; --ahead) {
+    for (int n = 0; n < (1 << 20) && !mbar_test(&full[done.st], done.phase); ++n) {
+    }
+    done.next(d.A);
+  }
+}
+
+// Fetches the lines that the block's first owner needs -- the previous
+// block's last owner's, or the halo -- into the first ring.
+template <int K>
+__device__ void fetch_mail(const SweepArgs& a, double* ring, int lane) {
+  using Geo = LineGeo<K>;
+  const Dir& d = a.d;
+  const long long so = d.chain1 ? d.s2 : d.s1;
+  int sl = 0;
+  for (int b = blockIdx.x * Geo::G; b < d.B; b += gridDim.x * Geo::G) {
+    for (int ch = 0; ch < d.A; ++ch) {
+      double v[K];
+      if (b == 0) {
+        const double* p = a.phi + d.base + ch * d.sa - so;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const int e = lane * K + k;
+          v[k] = e < d.L ? __ldcg(p + e * d.se) : 0.0;
+        }
+      } else {
+        double* slot = a.mail + ((long long)(b / Geo::G) * d.A + ch) * Geo::W;
+        Patience w;
+        for (;;) {
+          bool got = true;
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            v[k] = ld_relaxed_f64(slot + k * 32 + lane);
+            got = got && !is_empty(v[k]);
+          }
+          if (__all_sync(kAllLanes, got)) break;
+          if (w.gives_up(a.err, a.timeout_ns)) return;
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) st_relaxed_f64(slot + k * 32 + lane, empty_slot());
+      }
+      double* to = ring + (size_t)sl * Geo::W;
+      sl = sl + 1 == Geo::kSlots ? 0 : sl + 1;
+      Patience w;
+      for (;;) {
+        bool free = true;
+#pragma unroll
+        for (int k = 0; k < K; ++k) free = free && is_empty(ld_volatile_f64(to + k * 32 + lane));
+        if (__all_sync(kAllLanes, free)) break;
+        if (w.gives_up(a.err, a.timeout_ns)) return;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) st_volatile_f64(to + k * 32 + lane, v[k]);
+    }
+  }
+}
+
+// One lane's segment of the forward recurrence from the entering value, in
+// the sequential operations (division by the stored reciprocal and one
+// correction, which is the correctly rounded quotient: recipdiv.cuh). A
+// segment with an operand outside its range, or a numerator of -0 (the
+// correction would turn it into +0), is redone with `/`; the empty asm keeps
+// that division in a branch of its own (speculated, it doubled a pass).
+template <int K>
+__device__ __forceinline__ double forward_segment(const double (&dd)[K], const double (&lo)[K],
+                                                  const double (&m)[K], const double (&y)[K],
+                                                  bool y_ok, double in, double (&dp)[K]) {
+  bool ok = y_ok;
+  double p = in;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const double t = dd[k] - lo[k] * p;
+    const double q = t * y[k];
+    p = __fma_rn(__fma_rn(-q, m[k], t), y[k], q);
+    ok = ok && (__double_as_longlong(t) == 0 || exp_in_safe_range(t));
+    dp[k] = p;
+  }
+  if (!ok) {
+    asm volatile("" ::: "memory");
+    p = in;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      p = (dd[k] - lo[k] * p) / m[k];
+      dp[k] = p;
+    }
+  }
+  return p;
+}
+
+template <int K>
+__device__ __forceinline__ double backward_segment(const double (&dp)[K], const double (&cp)[K],
+                                                   double in, double (&x)[K]) {
+  double p = in;
+#pragma unroll
+  for (int k = K - 1; k >= 0; --k) {
+    p = dp[k] - cp[k] * p;
+    x[k] = p;
+  }
+  return p;
+}
+
+// Passes run before the first look at the fixed point, from the scan steps
+// that the line needs (a measure of its segments' contraction): the scan
+// leaves a few ulps, which two passes absorb where a segment contracts by
+// 2^-7 or more.
+__device__ __forceinline__ int first_passes(int scan_steps) {
+  return scan_steps <= 3 ? 2 : scan_steps;
+}
+
+template <int K, bool CHAIN1>
+__device__ void solve_lines(const SweepArgs& a, int w, double* bufs, uint64_t* full,
+                            uint64_t* empty, double* ring, double* next_ring, int lane) {
+  using Geo = LineGeo<K>;
+  const Dir& d = a.d;
+  const long long sc = CHAIN1 ? d.s1 : d.s2;
+  const int last_lane = (d.L - 1) / K;
+  int sl = 0;
+  double x[K];
+  for (LineAt<K> at(w); at.b < d.B; at.next(d.A)) {
+    const bool feeds = at.b + 1 < d.B;
+    const bool in_block = w + 1 < Geo::G;
+    if (at.ch == 0) {  // the chain starts from the halo
+      const double* p = a.phi + d.base + at.b * d.sb - sc;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int e = lane * K + k;
+        x[k] = e < d.L ? __ldcg(p + e * d.se) : 0.0;
+      }
+    }
+    const bool here = mbar_wait(&full[at.st], at.phase, a.err, a.timeout_ns);
+    if (!__all_sync(kAllLanes, here)) return;
+    double* buf = bufs + (size_t)at.st * Geo::kBuf;
+    auto op = [buf, lane](int arr, int k) { return buf[arr * Geo::W + k * 32 + lane]; };
+    double lo[K], m[K], y[K], cp[K], dd[K], t2[K];
+    bool y_ok = true;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      lo[k] = op(kRLo, k);
+      m[k] = op(kRM, k);
+      y[k] = op(kRY, k);
+      cp[k] = op(kRCp, k);
+      y_ok = y_ok && y[k] != 0.0;
+    }
+    const double end0 = buf[Geo::kScalars + kRE0] * buf[Geo::kEnds];
+    const double end1 = buf[Geo::kScalars + kRE1] * buf[Geo::kEnds + 1];
+    const int nf = (int)buf[Geo::kScalars + kRNf], nb = (int)buf[Geo::kScalars + kRNb];
+    double sf[kScanSteps], sb[kScanSteps];
+#pragma unroll
+    for (int s = 0; s < kScanSteps; ++s) {
+      sf[s] = buf[Geo::kScanF + 32 * s + lane];
+      sb[s] = buf[Geo::kScanB + 32 * s + lane];
+    }
+    double* to = next_ring + (size_t)sl * Geo::W;
+    if (!take_slot<K>(a, ring + (size_t)sl * Geo::W, feeds && in_block ? to : nullptr, lane, t2))
+      return;
+    sl = sl + 1 == Geo::kSlots ? 0 : sl + 1;
+    // right-hand side, the reference's order; the lagged couplings of the
+    // segment ends come last (:299-302, :325-328, :352-355)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int e = lane * K + k;
+      const double n1 = CHAIN1 ? x[k] : t2[k], n2 = CHAIN1 ? t2[k] : x[k];
+      double t = op(kRSu, k) + op(kR1m, k) * n1;
+      t = t + op(kR1p, k) * buf[Geo::kP1 + k * 32 + lane];
+      t = t + op(kR2m, k) * n2;
+      t = t + op(kR2p, k) * buf[Geo::kP2 + k * 32 + lane];
+      if (e == 0) t = t + end0;
+      if (e == d.L - 1) t = t + end1;
+      dd[k] = t;
+    }
+    // Forward: entering values from the scan, then the passes.
+    double dp[K];
+    double u = 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) u = __fma_rn(-lo[k] * y[k], u, dd[k] * y[k]);
+#pragma unroll
+    for (int s = 0; s < kScanSteps; ++s)
+      if (s < nf) u = __fma_rn(sf[s], __shfl_up_sync(kAllLanes, u, 1 << s), u);
+    auto enter_f = [lane](double out) {
+      const double v = __shfl_up_sync(kAllLanes, out, 1);
+      return lane == 0 ? 0.0 : v;
+    };
+    double inf = enter_f(u), nin = inf;
+    for (int n = first_passes(nf); n > 0; --n) {
+      inf = nin;
+      nin = enter_f(forward_segment<K>(dd, lo, m, y, y_ok, inf, dp));
+    }
+    bool settled = same_bits(nin, inf);
+    inf = nin;
+    // Backward, likewise; padding elements enter it as zeros whatever the
+    // forward passes left in them (0 * Inf), so the last element is dp itself.
+    auto clear_pads = [&] {
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (lane * K + k >= d.L) dp[k] = 0.0;
+    };
+    clear_pads();
+    u = 0.0;
+#pragma unroll
+    for (int k = K - 1; k >= 0; --k) u = __fma_rn(-cp[k], u, dp[k]);
+#pragma unroll
+    for (int s = 0; s < kScanSteps; ++s)
+      if (s < nb) u = __fma_rn(sb[s], __shfl_down_sync(kAllLanes, u, 1 << s), u);
+    auto enter_b = [lane, last_lane](double out) {
+      const double v = __shfl_down_sync(kAllLanes, out, 1);
+      return lane >= last_lane ? 0.0 : v;
+    };
+    double inb = enter_b(u);
+    nin = inb;
+    for (int n = first_passes(nb); n > 0; --n) {
+      inb = nin;
+      nin = enter_b(backward_segment<K>(dp, cp, inb, x));
+    }
+    settled = settled && same_bits(nin, inb);
+    inb = nin;
+    if (!__all_sync(kAllLanes, settled)) {  // on to the fixed points, each at most 32 passes away
+      for (int n = 0; n <= 32; ++n) {
+        nin = enter_f(forward_segment<K>(dd, lo, m, y, y_ok, inf, dp));
+        if (__all_sync(kAllLanes, same_bits(nin, inf))) break;
+        inf = nin;
+      }
+      clear_pads();
+      for (int n = 0; n <= 32; ++n) {
+        nin = enter_b(backward_segment<K>(dp, cp, inb, x));
+        if (__all_sync(kAllLanes, same_bits(nin, inb))) break;
+        inb = nin;
+      }
+    }
+    if (feeds && in_block) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) st_volatile_f64(to + k * 32 + lane, x[k]);
+    } else if (feeds) {
+      double* mail = a.mail + ((long long)((at.b + 1) / Geo::G) * d.A + at.ch) * Geo::W;
+#pragma unroll
+      for (int k = 0; k < K; ++k) st_relaxed_f64(mail + k * 32 + lane, x[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) buf[Geo::kP1 + k * 32 + lane] = x[k];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[at.st]);
+  }
+}
+
+// Warps 0..G-1 solve, G..2G-1 load and write, 2G fetches the mail. A warp whose wait
+// gave up leaves; the others' waits see the error word and leave too.
+template <int K, bool CHAIN1>
+__global__ void __launch_bounds__(LineGeo<K>::kThreads, 1) tdma_sweep_kernel(SweepArgs a) {
+  using Geo = LineGeo<K>;
+  extern __shared__ __align__(128) double sm[];
+  __shared__ __align__(8) uint64_t full[Geo::G][Geo::NB], empty[Geo::G][Geo::NB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* rings = sm + (size_t)Geo::G * Geo::NB * Geo::kBuf;
+  for (int i = threadIdx.x; i < Geo::G * Geo::kSlots * Geo::W; i += Geo::kThreads)
+    rings[i] = empty_slot();
+  // padding elements' neighbour values are never loaded
+  for (int i = threadIdx.x; i < Geo::G * Geo::NB * 2 * Geo::W; i += Geo::kThreads)
+    sm[(size_t)(i / (2 * Geo::W)) * Geo::kBuf + Geo::kP1 + i % (2 * Geo::W)] = 0.0;
+  if (threadIdx.x == 0) {
+    for (int g = 0; g < Geo::G; ++g)
+      for (int n = 0; n < Geo::NB; ++n) {
+        mbar_init(&full[g][n], 33);  // the bulk copy's expect and 32 lanes' copies
+        mbar_init(&empty[g][n], 1);
+      }
+    mbar_fence_init();
+  }
+  __syncthreads();
+  if (warp < Geo::G) {
+    solve_lines<K, CHAIN1>(a, warp, sm + (size_t)warp * Geo::NB * Geo::kBuf, full[warp],
+                           empty[warp], rings + (size_t)warp * Geo::kSlots * Geo::W,
+                           rings + (size_t)(warp + 1) * Geo::kSlots * Geo::W, lane);
+  } else if (warp < 2 * Geo::G) {
+    const int w = warp - Geo::G;
+    load_lines<K>(a, w, sm + (size_t)w * Geo::NB * Geo::kBuf, full[w], empty[w], lane);
+  } else {
+    fetch_mail<K>(a, rings, lane);
   }
 }
 
@@ -533,63 +856,176 @@ __global__ void div_check_kernel(long long n, unsigned long long seed,
   atomicAdd(counts + 1, fast);
 }
 
+// Elements per lane of a line of L: the next instantiated size.
+int line_k(int L) {
+  const int k = (L + 31) / 32;
+  return k <= 8 ? k : k <= 12 ? 12 : k <= 16 ? 16 : k <= 24 ? 24 : 32;
+}
+
+template <class F>
+auto with_k(int k, F f) {
+  switch (k) {
+    case 1: return f(std::integral_constant<int, 1>());
+    case 2: return f(std::integral_constant<int, 2>());
+    case 3: return f(std::integral_constant<int, 3>());
+    case 4: return f(std::integral_constant<int, 4>());
+    case 5: return f(std::integral_constant<int, 5>());
+    case 6: return f(std::integral_constant<int, 6>());
+    case 7: return f(std::integral_constant<int, 7>());
+    case 8: return f(std::integral_constant<int, 8>());
+    case 12: return f(std::integral_constant<int, 12>());
+    case 16: return f(std::integral_constant<int, 16>());
+    case 24: return f(std::integral_constant<int, 24>());
+    default: return f(std::integral_constant<int, 32>());
+  }
+}
+
+// The three directions' geometry (r, theta, z lines). The chain of the r and
+// z lines is theta; the theta lines' chain is the longer of r and z, since a
+// hand-over between owners costs more than a step along the chain.
+Dir make_dir(const HaloInputs& in, int nr, int nth, int nz, int dir) {
+  const long long sx = nr + 4, sxy = sx * (nth + 4);
+  Dir d;
+  d.base = 2 + 2 * sx + 2 * sxy;  // cell (1, 1, 1)
+  d.aP = in.aP;
+  d.Su = in.Su;
+  d.sx = sx;
+  d.wrap = dir == 1 ? 2 : 1;
+  d.b_fast = false;
+  d.chain1 = true;
+  if (dir == 0) {
+    d.A = nth; d.B = nz; d.L = nr;
+    d.sa = sx; d.sb = sxy; d.se = 1;
+    d.s1 = sx; d.c1m = in.aS; d.c1p = in.aN;
+    d.s2 = sxy; d.c2m = in.aB; d.c2p = in.aT;
+    d.lm = in.aW; d.lp = in.aE;
+  } else if (dir == 1) {
+    d.L = nth;
+    d.se = sx;
+    d.s1 = 1; d.c1m = in.aW; d.c1p = in.aE;
+    d.s2 = sxy; d.c2m = in.aB; d.c2p = in.aT;
+    d.lm = in.aS; d.lp = in.aN;
+    d.chain1 = nr >= nz;
+    d.A = d.chain1 ? nr : nz; d.B = d.chain1 ? nz : nr;
+    d.sa = d.chain1 ? 1 : sxy; d.sb = d.chain1 ? sxy : 1;
+    d.b_fast = !d.chain1;
+  } else {
+    d.A = nth; d.B = nr; d.L = nz;
+    d.sa = sx; d.sb = 1; d.se = sxy;
+    d.s1 = sx; d.c1m = in.aS; d.c1p = in.aN;
+    d.s2 = 1; d.c2m = in.aW; d.c2p = in.aE;
+    d.lm = in.aB; d.lp = in.aT;
+    d.b_fast = true;
+  }
+  return d;
+}
+
+struct DirSizes {
+  size_t rec, mail;  // doubles
+  int blocks, threads;
+};
+
+DirSizes dir_sizes(const Dir& d) {
+  return with_k(line_k(d.L), [&d](auto k) {
+    using Geo = LineGeo<decltype(k)::value>;
+    const int blocks = (d.B + Geo::G - 1) / Geo::G;
+    return DirSizes{(size_t)d.A * d.B * Geo::kRec, (size_t)blocks * d.A * Geo::W, blocks,
+                    Geo::kThreads};
+  });
+}
+
+template <int K, bool CHAIN1>
+cudaError_t launch_sweep(const SweepArgs& a, int sms, cudaStream_t st) {
+  using Geo = LineGeo<K>;
+  const void* k = (const void*)tdma_sweep_kernel<K, CHAIN1>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)Geo::kSmem);
+  if (e != cudaSuccess) return e;
+  // One block per SM; further owners follow in rounds.
+  const int blocks = (a.d.B + Geo::G - 1) / Geo::G;
+  SweepArgs copy = a;
+  void* args[] = {&copy};
+  return cudaLaunchCooperativeKernel(k, dim3(blocks < sms ? blocks : sms), dim3(Geo::kThreads),
+                                     args, Geo::kSmem, st);
+}
+
 }  // namespace
 
 size_t tdma_mailbox_doubles(int nr, int nth, int nz) {
-  return (size_t)6 * nr * nth * nz;
-}
-
-int tdma_grid(int nr, int nth, int nz) {
-  // Owners per direction: k (r lines), k (theta lines), i (z lines).
-  return nz > nr ? nz : nr;
+  size_t most = 0;
+  for (int dir = 0; dir < 3; ++dir) {
+    const size_t n = dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir)).mail;
+    if (n > most) most = n;
+  }
+  return most;
 }
 
 size_t tdma_factor_doubles(int nr, int nth, int nz) {
-  return (size_t)9 * nr * nth * nz;
+  size_t sum = 0;
+  for (int dir = 0; dir < 3; ++dir)
+    sum += dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir)).rec;
+  return sum;
+}
+
+void tdma_launch_shape(int nr, int nth, int nz, int sms, int* grid, int* block) {
+  *grid = 1;
+  *block = 1;
+  for (int dir = 0; dir < 3; ++dir) {
+    const DirSizes s = dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir));
+    if (s.blocks > *grid) *grid = s.blocks;
+    if (s.threads > *block) *block = s.threads;
+  }
+  if (*grid > sms) *grid = sms;
 }
 
 cudaError_t launch_tdma_f64(const HaloInputs& in, double* phi, int nr, int nth, int nz,
-                            int n_sweep, double* mbox, double* fac, const GroupWs& ws,
+                            int n_sweep, double* mbox, double* fac, int sms, const GroupWs& ws,
                             uint64_t timeout_ns, cudaStream_t st) {
   if (nr > kTdmaMaxLine || nth > kTdmaMaxLine || nz > kTdmaMaxLine)
     return cudaErrorInvalidValue;
-  TdmaArgs a;
-  a.in = in;
-  a.phi = phi;
-  a.nr = nr;
-  a.nth = nth;
-  a.nz = nz;
-  a.sx = nr + 4;
-  a.sxy = (long long)(nr + 4) * (nth + 4);
-  a.n_sweep = n_sweep;
-  int lmax = nr > nth ? nr : nth;
-  if (nz > lmax) lmax = nz;
-  a.lmax = lmax;
-  a.mbox = mbox;
-  a.fac = fac;
-  a.ws = ws;
-  a.timeout_ns = timeout_ns;
-  const int grid = tdma_grid(nr, nth, nz);
-  const size_t smem = (size_t)(2 * kBufArrays + 3) * lmax * sizeof(double);
   std::lock_guard<std::mutex> attr_lock(launch_attr_mutex());
-  cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024)
-    e = cudaFuncSetAttribute((const void*)tdma_kernel,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) {
-    const long long lines = (long long)nth * nz + (long long)nr * nz + (long long)nr * nth;
-    const int fb = 128;
-    long long fg = (lines + fb - 1) / fb;
-    if (fg > 4096) fg = 4096;
-    tdma_factor_kernel<<<(unsigned)fg, fb, 0, st>>>(a);
-    e = cudaGetLastError();
+  (void)cudaGetLastError();  // report these launches' errors, not an older one
+  const double* rec[3];
+  for (int dir = 0; dir < 3; ++dir) {
+    FactorArgs f;
+    f.d = make_dir(in, nr, nth, nz, dir);
+    f.rec = fac;
+    f.mail = mbox;
+    f.phi = dir == 0 ? phi : nullptr;
+    f.err = dir == 0 ? ws.err : nullptr;
+    f.nr = nr;
+    f.nth = nth;
+    f.nz = nz;
+    rec[dir] = fac;
+    fac += dir_sizes(f.d).rec;
+    const long long lines = (long long)f.d.A * f.d.B;
+    long long grid = (lines + kFactorBlock / 32 - 1) / (kFactorBlock / 32);
+    if (grid > 8LL * sms) grid = 8LL * sms;
+    with_k(line_k(f.d.L), [&](auto k) {
+      tdma_factor_kernel<decltype(k)::value><<<(unsigned)grid, kFactorBlock, 0, st>>>(f);
+      return 0;
+    });
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.counter, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  void* args[] = {&a};
-  return cudaLaunchCooperativeKernel((const void*)tdma_kernel, dim3(grid), dim3(kTdmaBlock), args,
-                                     smem, st);
+  for (int sweep = 1; sweep <= n_sweep; ++sweep) {
+    for (int dir = 0; dir < 3; ++dir) {
+      SweepArgs a;
+      a.d = make_dir(in, nr, nth, nz, dir);
+      if (dir == 2 && sweep == n_sweep) a.d.wrap = 0;  // no refresh after the last direction
+      a.rec = rec[dir];
+      a.mail = mbox;
+      a.phi = phi;
+      a.err = ws.err;
+      a.timeout_ns = timeout_ns;
+      const cudaError_t e = with_k(line_k(a.d.L), [&](auto k) {
+        constexpr int K = decltype(k)::value;
+        return a.d.chain1 ? launch_sweep<K, true>(a, sms, st) : launch_sweep<K, false>(a, sms, st);
+      });
+      if (e != cudaSuccess) return e;
+    }
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_residual_f64(const HaloInputs& in, const double* phi, const MeshDims& d,
@@ -611,7 +1047,6 @@ cudaError_t launch_residual_f64(const HaloInputs& in, const double* phi, const M
                                      args, 0, st);
 }
 
-const void* tdma_kernel_ptr() { return (const void*)tdma_kernel; }
 const void* residual_kernel_ptr() { return (const void*)residual_kernel; }
 
 cudaError_t run_div_check(long long n, unsigned long long seed, unsigned long long* counts,
