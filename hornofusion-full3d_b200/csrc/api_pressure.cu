@@ -39,7 +39,7 @@ int enqueue_tdma(eaf_cg* h, const HaloInputs& in, double* phi, int n_sweep) {
   }
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(cudaEventRecord(h->ev[4], h->st));
-  h->last_kernels = n_sweep > 0 ? 3 + 3 * n_sweep : 0;
+  h->last_kernels = n_sweep > 0 ? 3 + 6 * n_sweep : 0;
   return EAF_OK;
 }
 

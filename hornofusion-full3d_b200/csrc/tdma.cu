@@ -17,33 +17,39 @@
 // its own signal (slots hold a signalling NaN, which arithmetic never
 // produces, until written, and the consumer marks them empty again). G
 // adjacent owners share a block and hand over through shared memory; only
-// every G-th hand-over crosses blocks, through global memory (the mail warp
-// of the consuming block fetches it ahead of the solver). A loader warp per
-// solver copies the next lines' operands into a ring of buffers. The owner is
+// every G-th hand-over crosses blocks, through global memory (the consuming
+// block's mail warp fetches it ahead of the solver). A loader warp per solver
+// copies the next lines' operands into a ring of buffers and writes the
+// solved lines to phi. The owner is
 // the shorter of the two line indices, never theta (its periodic halo must
 // keep the old values until its chain ends).
 //
 // A line solve. Both halves of the Thomas solve that depend on phi,
 //   dp_i = (d_i - a_i dp_{i-1}) / m_i,   x_i = dp_i - cp_i x_{i+1},
 // are first-order recurrences of correctly rounded operations, sequential in
-// i. One lane running them took 95 ns an element, all of it latency. Here
-// each lane owns K = ceil(L/32) consecutive elements and needs only the
-// value entering its segment. A prefix scan of the segments' affine maps
-// gives that to a few ulps; then every lane runs its segment with the
-// sequential operations and hands its last value on, and the warp repeats
-// until no entering value changes by a single bit. Then, by induction from
-// lane 0, whose input is exact, every value is the sequential recurrence's,
-// whatever the scan delivered. Two passes are the rule, because a segment
-// contracts an error of a few ulps below a rounding; a line without
-// contraction takes up to 32, about the sequential cost. Per line of 120
-// elements the recurrences are 2 x 8 dependent elements long instead of
-// 2 x 120.
+// i. One lane running them took 95 ns an element, all of it latency. Here a
+// lane owns K consecutive elements and needs only the value entering its
+// segment. A prefix scan of the segments' affine maps gives that to a few
+// ulps; then every lane runs its segment with the sequential operations and
+// hands its last value on, and the warp repeats until no entering value
+// changes by a single bit. Then, by induction from lane 0, whose input is
+// exact, every value is the sequential recurrence's, whatever the scan
+// delivered. Two passes are the rule, because a segment contracts an error of
+// a few ulps below a rounding; a line without contraction takes up to 32,
+// about the sequential cost. A pass costs 42 cycles an element (five
+// dependent FP64 operations) plus a shuffle, so the passes needed times K is
+// what counts: K = 4 on as few lanes as the line fills, more only beyond 128
+// elements (one element a lane needs four to five passes and five scan steps).
 //
-// What does not depend on phi -- the guarded pivots m_i, cp_i, y_i = 1/m_i
-// and the scan's segment products -- is computed once per call, by the same
-// fixed-point passes, in a record per line and direction that also holds the
-// line's coefficients in the order the solver's lanes read them, so a line
-// is one bulk copy plus the old neighbour values.
+// Layout. The sweep itself is bound by latency, so the transposing work is
+// left to parallel kernels before it: what does not depend on phi -- the
+// guarded pivots m_i, cp_i, y_i = 1/m_i (by the same fixed-point passes) and
+// the scan's segment products -- is computed once per call into a record per
+// line and direction, lane by lane; what a direction takes from the old phi
+// (its plus-side neighbours, which no line changes before it is solved) goes
+// into an old-value record per line before each direction. A line is then two
+// bulk copies. (Gathering the old values in the sweep cost a third of it:
+// every element of a theta or z line is a sector of its own.)
 // Built with -fmad=false like the CG unit.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -68,39 +74,63 @@ __device__ __forceinline__ double sign_small(double v) {
 constexpr int kTdmaMaxLine = 1024;
 constexpr unsigned kAllLanes = 0xffffffffu;
 
-// Record of one line: nine arrays of W = 32 K doubles, element lane*K + k of
-// the line at [k][lane]; the scan's products, [step][lane], forward then
-// backward; four scalars.
-enum { kRSu, kR1m, kR1p, kR2m, kR2p, kRLo, kRM, kRY, kRCp, kRArrays };
+// Record of one line: four scalars, then per lane seven arrays of its K
+// elements and the scan's products, forward and backward in turn. K is even
+// and the lane strides are 2 mod 4, so that the lanes read 16 bytes at a time
+// without bank conflicts.
+enum { kRSu, kR1m, kR2m, kRLo, kRM, kRY, kRCp, kRArrays };
 constexpr int kScanSteps = 5;
-enum { kRE0, kRE1, kRNf, kRNb, kRScalars };  // end links, scan steps needed
+enum { kRE0, kRE1, kRNf, kRNb, kRScalars };  // end links, scan steps needed (and kUnsafe)
+// Old values of one line: the two halo values beyond its ends (and two words
+// of padding), then per lane the products of the plus-side neighbours of pairs
+// 1 and 2 and the coupling of the line's far end (-0.0 elsewhere).
+enum { kO1 = 0, kO2 = 1, kOEnd = 2, kOArrays = 3, kOScalars = 4 };
+constexpr int kUnsafe = 8;  // added to the forward steps: a pivot outside the reciprocal's range
 
-// Sizes for K elements a lane: owners per block, operand buffers per owner
-// and hand-over slots per ring, as many as 220 KB of shared memory hold (at
-// least three buffers before a further owner).
+constexpr int lane_stride(int doubles) { return doubles + (6 - doubles % 4) % 4; }
+
 template <int K>
-struct LineGeo {
-  static constexpr int W = 32 * K;
-  static constexpr int kScanF = kRArrays * W;
-  static constexpr int kScanB = kScanF + 32 * kScanSteps;
-  static constexpr int kScalars = kScanB + 32 * kScanSteps;
-  static constexpr int kRec = kScalars + kRScalars;
-  static constexpr int kP1 = kRec, kP2 = kRec + W, kEnds = kRec + 2 * W;
-  static constexpr int kBuf = kEnds + 4;
-  static constexpr int kSlots = K <= 16 ? 4 : 2;
-  static constexpr int kLimit = 220 * 1024 / 8;
-  static constexpr int need(int g, int nb) { return g * (nb * kBuf + kSlots * W); }
-  static constexpr int owners() {
-    for (int g = 8; g > 1; --g)
-      if ((g <= 4 || K <= 2) && need(g, 3) <= kLimit) return g;
-    return 1;
-  }
-  static constexpr int G = owners();
-  static constexpr int NB = need(G, 4) <= kLimit ? 4 : need(G, 3) <= kLimit ? 3 : 2;
-  static constexpr int kThreads = 32 * (2 * G + 1);
-  static constexpr size_t kSmem = (size_t)need(G, NB) * sizeof(double);
-  static_assert(need(G, NB) <= kLimit, "line buffers exceed the shared memory");
+struct Lanes {
+  static_assert(K % 2 == 0, "16-byte reads");
+  static constexpr int kScan = kRArrays * K;
+  static constexpr int kRec = lane_stride(kScan + 2 * kScanSteps);  // in a record
+  static constexpr int kOld = lane_stride(kOArrays * K);  // in old values
+  static constexpr int kRing = lane_stride(K);     // of a hand-over slot
+  static constexpr int kMail = 32 * K;             // slot between blocks
+  // One owner per scheduler; long lines leave registers for fewer.
+  static constexpr int kMaxOwners = K <= 8 ? 4 : K <= 16 ? 2 : 1;
+  static constexpr int kMaxThreads = 32 * (2 * kMaxOwners + 1);
 };
+
+// Sizes for lines of L elements (doubles): lanes in use, record, old values,
+// buffer (both), and owners per block, buffers per owner and hand-over slots
+// per ring, as many as 220 KB of shared memory hold (three buffers before a
+// further owner).
+struct LineGeo {
+  int n, rec, old, buf, G, NB, slots, ring;
+  size_t smem;
+};
+
+template <int K>
+LineGeo line_geo(int L) {
+  using Ln = Lanes<K>;
+  constexpr int limit = 220 * 1024 / 8;
+  LineGeo g;
+  g.n = (L + K - 1) / K;
+  g.rec = (kRScalars + g.n * Ln::kRec + 1) & ~1;
+  g.old = kOScalars + g.n * Ln::kOld;
+  g.buf = g.rec + g.old;  // (all even: 16-byte copies and reads)
+  g.ring = 32 * Ln::kRing;
+  g.slots = K <= 16 ? 4 : 2;
+  auto need = [&g](int owners, int nb) {
+    return owners * (nb * g.buf + g.slots * g.ring) + Ln::kRec + Ln::kOld;
+  };
+  g.G = Ln::kMaxOwners;
+  while (g.G > 1 && need(g.G, 3) > limit) --g.G;
+  g.NB = need(g.G, 4) <= limit ? 4 : need(g.G, 3) <= limit ? 3 : 2;
+  g.smem = (size_t)need(g.G, g.NB) * sizeof(double);
+  return g;
+}
 
 // One direction. Cell (a, b, e) sits at halo index base + a*sa + b*sb + e*se;
 // pair 1 and pair 2 are the neighbour pairs of the right-hand side
@@ -119,6 +149,8 @@ struct Dir {
 
 struct FactorArgs {
   Dir d;
+  LineGeo g;
+  int tile;           // lines per block
   double* rec;
   double* mail;       // hand-over slots between blocks, marked empty here
   double* phi;        // non-null: refresh the theta halos (first direction)
@@ -126,9 +158,18 @@ struct FactorArgs {
   int* err;
 };
 
+struct OldArgs {
+  Dir d;
+  LineGeo g;
+  int tile;
+  const double* phi;
+  double* old;
+};
+
 struct SweepArgs {
   Dir d;
-  const double* rec;
+  LineGeo g;
+  const double *rec, *old;
   double* mail;
   double* phi;
   int* err;
@@ -136,14 +177,10 @@ struct SweepArgs {
 };
 
 // Empty hand-over slot: a signalling NaN (IEEE arithmetic only delivers
-// quiet NaNs, so no solution value has this pattern).
-constexpr unsigned long long kEmptyBits = 0x7ff000017ff00001ull;
-__device__ __forceinline__ double empty_slot() {
-  return __longlong_as_double((long long)kEmptyBits);
-}
-__device__ __forceinline__ bool is_empty(double v) {
-  return (unsigned long long)__double_as_longlong(v) == kEmptyBits;
-}
+// quiet NaNs, so no solution value has this high word).
+constexpr int kEmptyHigh = 0x7ff00001;
+__device__ __forceinline__ double empty_slot() { return __hiloint2double(kEmptyHigh, kEmptyHigh); }
+__device__ __forceinline__ bool is_empty(double v) { return __double2hiint(v) == kEmptyHigh; }
 __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
@@ -168,129 +205,252 @@ __device__ void theta_wrap(double* phi, int nr, int nth, int nz) {
 }
 
 // ---------------------------------------------------------------------------
-// Line records: one warp per line. The pivots' recurrence (:30-38)
+// Line records. A block builds the records of `tile` lines that are adjacent
+// in the unit-stride index (r lines: adjacent rows) in shared memory: all
+// threads gather the coefficients, neighbouring threads neighbouring
+// addresses, then a warp per line computes its factors in place, and one bulk
+// store writes each record. (A warp gathering its own line with strides of a
+// row or a plane between lanes was bound by its 32 sectors a load: 1280 us at
+// 120x240x168 against the bytes' 330.) The pivots' recurrence (:30-38)
 //   m_i = guard(b_i - a_i cp_{i-1}),  cp_i = c_i / m_i
 // runs in the lanes' segments from the previous pass's entering values until
 // none changes (the first pass starts from zero: the recurrence forgets its
 // start within a few elements). Padding elements and the line's ends carry
-// values that leave the solver's recurrences untouched: lo = 0 in the first
-// element, cp = 0 in the last, and m = y = 1 with zero links beyond.
-// Bound by its stores: 60x120x84, 200 MB of records.
+// values that leave the solver's recurrences untouched: cp = 0 in the last
+// element, and m = y = 1 with zero links beyond. The first element's lo takes
+// no part in the pivots: with it the solver adds the lagged coupling of the
+// line's near end (see solve_lines).
 // ---------------------------------------------------------------------------
-constexpr int kFactorBlock = 256;
+constexpr int kTileBlock = 256;
+
+// A block's lines: `tile` adjacent ones in the unit-stride line index u (r
+// lines: in the chain's) at one value v of the other.
+struct Tile {
+  int u0, v, lines;
+  __device__ Tile(const Dir& d, int tile) {
+    const int U = d.b_fast ? d.B : d.A;
+    const int tiles = (U + tile - 1) / tile;
+    u0 = (int)(blockIdx.x % tiles) * tile;
+    v = (int)(blockIdx.x / tiles);
+    lines = min(tile, U - u0);
+  }
+  __device__ __forceinline__ int a_of(const Dir& d, int u) const { return d.b_fast ? v : u0 + u; }
+  __device__ __forceinline__ int b_of(const Dir& d, int u) const { return d.b_fast ? u0 + u : v; }
+  // Halo index of element 0 of the tile's line u.
+  __device__ __forceinline__ long long cell(const Dir& d, int u) const {
+    return d.base + a_of(d, u) * d.sa + b_of(d, u) * d.sb;
+  }
+  // Work item t of lines x E elements, neighbouring items at neighbouring
+  // addresses.
+  __device__ __forceinline__ void split(const Dir& d, int t, int E, int& u, int& e) const {
+    u = d.se == 1 ? t / E : t % lines;
+    e = d.se == 1 ? t % E : t / lines;
+  }
+};
+
+__device__ __forceinline__ void bulk_copy_s2g(double* dst, const double* src, int bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+               "r"(smem_addr(src)), "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_copies_done() {
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 
 template <int K>
-__global__ void __launch_bounds__(kFactorBlock) tdma_factor_kernel(FactorArgs a) {
-  using Geo = LineGeo<K>;
+__device__ __forceinline__ void factor_line(const Dir& d, const LineGeo& g, double* rec,
+                                            int lane) {
+  using Ln = Lanes<K>;
+  double* r = rec + kRScalars + lane * Ln::kRec;
+  const bool on = lane < g.n;
+  double lo[K], bb[K], cc[K], mm[K], cp[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    lo[k] = on && lane + k > 0 ? r[kRLo * K + k] : 0.0;
+    bb[k] = on ? r[kRM * K + k] : 1.0;
+    cc[k] = on ? r[kRCp * K + k] : 0.0;
+  }
+  double in = 0.0;
+  for (int pass = 0; pass <= 32; ++pass) {
+    double c = in;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      mm[k] = sign_small(bb[k] - lo[k] * c);
+      c = cc[k] / mm[k];
+      cp[k] = c;
+    }
+    double nin = __shfl_up_sync(kAllLanes, c, 1);
+    if (lane == 0 || !on) nin = 0.0;
+    if (__all_sync(kAllLanes, same_bits(nin, in))) break;
+    in = nin;
+  }
+  double pf = on ? 1.0 : 0.0, pb = pf;
+  bool safe = true;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const bool in_range = exp_in_safe_range(mm[k]);
+    const double y = in_range ? 1.0 / mm[k] : 0.0;
+    safe = safe && in_range;
+    const double cpe = lane * K + k < d.L - 1 ? cp[k] : 0.0;
+    if (on) {
+      r[kRM * K + k] = mm[k];
+      r[kRY * K + k] = y;
+      r[kRCp * K + k] = cpe;
+    }
+    pf = pf * (-lo[k] * y);
+    pb = pb * -cpe;
+  }
+  // Scan products: step s adds the value 2^s lanes away times the product
+  // over the 2^s segments in between; a step whose products are all below
+  // 2^-56 (and those after it) would change nothing and is left out.
+  int nf = 0, nb = 0;
+#pragma unroll
+  for (int s = 0; s < kScanSteps; ++s) {
+    if (on) {
+      r[Ln::kScan + 2 * s] = pf;
+      r[Ln::kScan + 2 * s + 1] = pb;
+    }
+    if (nf == s && __any_sync(kAllLanes, !(fabs(pf) < 0x1p-56))) nf = s + 1;
+    if (nb == s && __any_sync(kAllLanes, !(fabs(pb) < 0x1p-56))) nb = s + 1;
+    pf = pf * __shfl_up_sync(kAllLanes, pf, 1 << s);
+    pb = pb * __shfl_down_sync(kAllLanes, pb, 1 << s);
+  }
+  safe = __all_sync(kAllLanes, safe);
+  if (lane == 0) {
+    rec[kRNf] = (double)(safe ? nf : nf + kUnsafe);
+    rec[kRNb] = (double)nb;
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kTileBlock) tdma_factor_kernel(FactorArgs a) {
+  using Ln = Lanes<K>;
+  extern __shared__ __align__(128) double sm[];
   const Dir& d = a.d;
-  const int lane = threadIdx.x & 31;
-  const long long lines = (long long)d.A * d.B;
-  const long long warps = (long long)gridDim.x * (kFactorBlock / 32);
+  const LineGeo& g = a.g;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (a.phi) theta_wrap(a.phi, a.nr, a.nth, a.nz);
   if (a.err && blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0;
-  for (long long t = (long long)blockIdx.x * (kFactorBlock / 32) + (threadIdx.x >> 5); t < lines;
-       t += warps) {
-    const int ch = d.b_fast ? (int)(t / d.B) : (int)(t % d.A);
-    const int b = d.b_fast ? (int)(t % d.B) : (int)(t / d.A);
-    const long long q0 = d.base + ch * d.sa + b * d.sb;
-    double* rec = a.rec + ((long long)b * d.A + ch) * Geo::kRec;
-    double lo[K], bb[K], cc[K], mm[K], cp[K];
+  const Tile tl(d, a.tile);
+  const int E = g.n * K;  // elements with padding
+  for (int t = threadIdx.x; t < tl.lines * E; t += kTileBlock) {
+    int u, e;
+    tl.split(d, t, E, u, e);
+    double* rec = sm + (size_t)u * g.rec;
+    double* r = rec + kRScalars + (e / K) * Ln::kRec + e % K;
+    if (e < d.L) {
+      const long long q = tl.cell(d, u) + e * d.se;
+      const double lm = d.lm[q], lp = d.lp[q], ap = d.aP[q], s0 = d.Su[q], c1m = d.c1m[q],
+                   c2m = d.c2m[q];
+      r[kRSu * K] = s0;
+      r[kR1m * K] = c1m;
+      r[kR2m * K] = c2m;
+      r[kRLo * K] = d.L > 1 ? -lm : 0.0;
+      r[kRM * K] = ap;
+      r[kRCp * K] = -lp;
+      if (e == 0) rec[kRE0] = lm;
+      if (e == d.L - 1) rec[kRE1] = lp;
+    } else {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int e = lane * K + k;
-      const long long q = q0 + e * d.se;
-      const bool live = e < d.L;
-      lo[k] = live && e > 0 ? -d.lm[q] : 0.0;
-      bb[k] = live ? d.aP[q] : 1.0;
-      cc[k] = live ? -d.lp[q] : 0.0;
+      for (int arr = 0; arr < kRArrays; ++arr) r[arr * K] = arr == kRM ? 1.0 : 0.0;
     }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int e = lane * K + k;
-      const long long q = q0 + e * d.se;
-      const bool live = e < d.L;
-      const int o = k * 32 + lane;
-      rec[kRSu * Geo::W + o] = live ? d.Su[q] : 0.0;
-      rec[kR1m * Geo::W + o] = live ? d.c1m[q] : 0.0;
-      rec[kR1p * Geo::W + o] = live ? d.c1p[q] : 0.0;
-      rec[kR2m * Geo::W + o] = live ? d.c2m[q] : 0.0;
-      rec[kR2p * Geo::W + o] = live ? d.c2p[q] : 0.0;
-    }
-    double in = 0.0;
-    for (int pass = 0; pass <= 32; ++pass) {
-      double c = in;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        mm[k] = sign_small(bb[k] - lo[k] * c);
-        c = cc[k] / mm[k];
-        cp[k] = c;
-      }
-      double nin = __shfl_up_sync(kAllLanes, c, 1);
-      if (lane == 0) nin = 0.0;
-      if (__all_sync(kAllLanes, same_bits(nin, in))) break;
-      in = nin;
-    }
-    double pf = 1.0, pb = 1.0;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int e = lane * K + k;
-      const int o = k * 32 + lane;
-      const double y = exp_in_safe_range(mm[k]) ? 1.0 / mm[k] : 0.0;
-      const double cpe = e < d.L - 1 ? cp[k] : 0.0;
-      rec[kRLo * Geo::W + o] = lo[k];
-      rec[kRM * Geo::W + o] = mm[k];
-      rec[kRY * Geo::W + o] = y;
-      rec[kRCp * Geo::W + o] = cpe;
-      pf = pf * (-lo[k] * y);
-      pb = pb * -cpe;
-    }
-    // Scan products: step s adds the value 2^s lanes away times the product
-    // over the 2^s segments in between; a step whose products are all below
-    // 2^-56 (and those after it) would change nothing and is left out.
-    int nf = 0, nb = 0;
-#pragma unroll
-    for (int s = 0; s < kScanSteps; ++s) {
-      rec[Geo::kScanF + 32 * s + lane] = pf;
-      rec[Geo::kScanB + 32 * s + lane] = pb;
-      if (nf == s && __any_sync(kAllLanes, !(fabs(pf) < 0x1p-56))) nf = s + 1;
-      if (nb == s && __any_sync(kAllLanes, !(fabs(pb) < 0x1p-56))) nb = s + 1;
-      pf = pf * __shfl_up_sync(kAllLanes, pf, 1 << s);
-      pb = pb * __shfl_down_sync(kAllLanes, pb, 1 << s);
-    }
-    if (lane == 0) {
-      double* sc = rec + Geo::kScalars;
-      sc[kRE0] = d.lm[q0];
-      sc[kRE1] = d.lp[q0 + (long long)(d.L - 1) * d.se];
-      sc[kRNf] = (double)nf;
-      sc[kRNb] = (double)nb;
-    }
-    if (b % Geo::G == 0) {
-      double* slot = a.mail + ((long long)(b / Geo::G) * d.A + ch) * Geo::W;
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the bulk stores
+  __syncthreads();
+  for (int u = warp; u < tl.lines; u += kTileBlock / 32) {
+    double* rec = sm + (size_t)u * g.rec;
+    const int ch = tl.a_of(d, u), b = tl.b_of(d, u);
+    factor_line<K>(d, g, rec, lane);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) bulk_copy_s2g(a.rec + ((long long)b * d.A + ch) * g.rec, rec, g.rec * 8);
+    if (b % g.G == 0) {
+      double* slot = a.mail + ((long long)(b / g.G) * d.A + ch) * Ln::kMail;
 #pragma unroll
       for (int k = 0; k < K; ++k) slot[k * 32 + lane] = empty_slot();
     }
+  }
+  if (lane == 0) bulk_copies_done();
+}
+
+// Old-value records of one direction, in the factor kernel's tiles.
+template <int K>
+__global__ void __launch_bounds__(kTileBlock) tdma_old_kernel(OldArgs a) {
+  using Ln = Lanes<K>;
+  extern __shared__ __align__(128) double sm[];
+  const Dir& d = a.d;
+  const LineGeo& g = a.g;
+  const Tile tl(d, a.tile);
+  const int E = g.n * K;
+  const double* __restrict__ phi = a.phi;
+  for (int t = threadIdx.x; t < tl.lines * E; t += kTileBlock) {
+    int u, e;
+    tl.split(d, t, E, u, e);
+    double* rec = sm + (size_t)u * g.old;
+    double* r = rec + kOScalars + (e / K) * Ln::kOld + e % K;
+    double o1 = 0.0, o2 = 0.0, end = -0.0;
+    if (e < d.L) {
+      const long long q = tl.cell(d, u) + e * d.se;
+      o1 = d.c1p[q] * phi[q + d.s1];
+      o2 = d.c2p[q] * phi[q + d.s2];
+      if (e == 0) rec[0] = phi[q - d.se];
+      if (e == d.L - 1) {
+        const double far = phi[q + d.se];
+        rec[1] = far;
+        if (d.L > 1) end = d.lp[q] * far;
+      }
+    }
+    r[kO1 * K] = o1;
+    r[kO2 * K] = o2;
+    r[kOEnd * K] = end;
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int u = 0; u < tl.lines; ++u)
+      bulk_copy_s2g(a.old + ((long long)tl.b_of(d, u) * d.A + tl.a_of(d, u)) * g.old,
+                    sm + (size_t)u * g.old, g.old * 8);
+    bulk_copies_done();
   }
 }
 
 // ---------------------------------------------------------------------------
 // Sweep of one direction.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double ld_volatile_f64(const double* p) {
-  return *(const volatile double*)p;
+// Shared memory by its 32-bit addresses: a solver's line is short of issue
+// slots, and generic 64-bit addresses cost it a third more instructions.
+using saddr = uint32_t;
+__device__ __forceinline__ void ld_pair(saddr p, double& v, double& w) {
+  asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v), "=d"(w) : "r"(p));
 }
-__device__ __forceinline__ void st_volatile_f64(double* p, double v) {
-  *(volatile double*)p = v;
+__device__ __forceinline__ void st_pair(saddr p, double v, double w) {
+  asm volatile("st.volatile.shared.v2.f64 [%0], {%1, %2};" ::"r"(p), "d"(v), "d"(w) : "memory");
 }
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src)
-               : "memory");
+template <int N>
+__device__ __forceinline__ void ld_pairs(saddr p, double (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) ld_pair(p + 8 * i, v[i], v[i + 1]);
 }
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
+template <int N>
+__device__ __forceinline__ void st_pairs(saddr p, const double (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) st_pair(p + 8 * i, v[i], v[i + 1]);
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+// (mbar_test may suspend the warp; this looks and returns)
+__device__ __forceinline__ bool mbar_look(saddr bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_arrive(saddr bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // Bound of a polling loop; warp-uniform, true when the wait gives up (the
@@ -314,30 +474,23 @@ struct Patience {
   }
 };
 
-// Takes this lane's K values of a hand-over slot in shared memory once all
-// have arrived, and marks them empty; with `next`, also waits until the lane's
-// values of that slot (the one this line goes to) have been taken.
+// A lane's K values in a hand-over slot in shared memory.
 template <int K>
-__device__ __forceinline__ bool take_slot(const SweepArgs& a, double* slot, const double* next,
-                                          int lane, double (&v)[K]) {
-  Patience w;
-  for (;;) {
-    bool ready = true;
+__device__ __forceinline__ bool slot_full(saddr slot, double (&v)[K]) {
+  ld_pairs(slot, v);
+  bool all = true;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      v[k] = ld_volatile_f64(slot + k * 32 + lane);
-      ready = ready && !is_empty(v[k]);
-    }
-    if (next) {
+  for (int k = 0; k < K; ++k) all = all & !is_empty(v[k]);
+  return all;
+}
+template <int K>
+__device__ __forceinline__ bool slot_free(saddr slot) {
+  double v[K];
+  ld_pairs(slot, v);
+  bool all = true;
 #pragma unroll
-      for (int k = 0; k < K; ++k) ready = ready && is_empty(ld_volatile_f64(next + k * 32 + lane));
-    }
-    if (__all_sync(kAllLanes, ready)) break;
-    if (w.gives_up(a.err, a.timeout_ns)) return false;
-  }
-#pragma unroll
-  for (int k = 0; k < K; ++k) st_volatile_f64(slot + k * 32 + lane, empty_slot());
-  return true;
+  for (int k = 0; k < K; ++k) all = all & is_empty(v[k]);
+  return all;
 }
 
 // Writes a solved line from its buffer to phi, and the theta halos that it
@@ -345,14 +498,14 @@ __device__ __forceinline__ bool take_slot(const SweepArgs& a, double* slot, cons
 // chain, at the chain's end, the owner's columns (their old halo values are
 // no longer needed; the lane reads back values that it wrote).
 template <int K>
-__device__ __forceinline__ void write_line(const SweepArgs& a, const double* buf, int b, int ch,
+__device__ __forceinline__ void write_line(const SweepArgs& a, const double* old, int b, int ch,
                                            int lane) {
-  using Geo = LineGeo<K>;
   const Dir& d = a.d;
+  if (lane >= a.g.n) return;
   double* p = a.phi + d.base + ch * d.sa + b * d.sb;
   double x[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) x[k] = buf[Geo::kP1 + k * 32 + lane];
+  for (int k = 0; k < K; ++k) x[k] = old[k];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int e = lane * K + k;
@@ -386,137 +539,123 @@ __device__ __forceinline__ void write_line(const SweepArgs& a, const double* buf
 }
 
 // Position of a warp in its owners' lines, with the buffer it is in.
-template <int K>
 struct LineAt {
   int b, ch = 0, st = 0;
   uint32_t phase = 0;
-  __device__ explicit LineAt(int w) : b(blockIdx.x * LineGeo<K>::G + w) {}
-  __device__ __forceinline__ void next(int A) {
-    if (++st == LineGeo<K>::NB) {
+  __device__ LineAt(const LineGeo& g, int w) : b(blockIdx.x * g.G + w) {}
+  __device__ __forceinline__ void next(const Dir& d, const LineGeo& g) {
+    if (++st == g.NB) {
       st = 0;
       phase ^= 1u;
     }
-    if (++ch == A) {
+    if (++ch == d.A) {
       ch = 0;
-      b += gridDim.x * LineGeo<K>::G;
+      b += gridDim.x * g.G;
     }
   }
 };
 
 // Copies the operands of the owner's lines into its ring of buffers, as far
 // ahead as the solver has finished with them, and writes each finished line
-// out of its buffer before that is filled again. The old neighbour values may
-// be read at any time before the line is solved: a line's plus-side
-// neighbours are solved, and written, after it.
+// out of its buffer before that is filled again.
 template <int K>
 __device__ void load_lines(const SweepArgs& a, int w, double* bufs, uint64_t* full,
                            uint64_t* empty, int lane) {
-  using Geo = LineGeo<K>;
+  using Ln = Lanes<K>;
   const Dir& d = a.d;
-  LineAt<K> at(w), done(w);
+  const LineGeo& g = a.g;
+  LineAt at(g, w), done(g, w);
   int ahead = 0;  // lines issued and not yet written out
-  bool ok = true;
-  while (ok && done.b < d.B) {
-    if (ahead == Geo::NB || at.b >= d.B) {
-      ok = mbar_wait(&empty[done.st], done.phase, a.err, a.timeout_ns);
-      ok = __all_sync(kAllLanes, ok);
-      if (!ok) break;
-      write_line<K>(a, bufs + (size_t)done.st * Geo::kBuf, done.b, done.ch, lane);
-      done.next(d.A);
-      --ahead;
-    }
-    if (at.b >= d.B) continue;
-    double* buf = bufs + (size_t)at.st * Geo::kBuf;
-    const double* p = a.phi + d.base + at.ch * d.sa + at.b * d.sb;
-    if (lane == 0) {
-      mbar_arrive_expect(&full[at.st], Geo::kRec * 8);
-      bulk_copy_g2s(buf, a.rec + ((long long)at.b * d.A + at.ch) * Geo::kRec, Geo::kRec * 8,
-                    &full[at.st]);
-      cp_async8(buf + Geo::kEnds, p - d.se);
-      cp_async8(buf + Geo::kEnds + 1, p + d.L * d.se);
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int e = lane * K + k;
-      if (e < d.L) {
-        cp_async8(buf + Geo::kP1 + k * 32 + lane, p + e * d.se + d.s1);
-        cp_async8(buf + Geo::kP2 + k * 32 + lane, p + e * d.se + d.s2);
+  Patience wait;
+  while (done.b < d.B) {
+    if (ahead < g.NB && at.b < d.B) {
+      if (lane == 0) {
+        const long long line = (long long)at.b * d.A + at.ch;
+        double* buf = bufs + (size_t)at.st * g.buf;
+        mbar_arrive_expect(&full[at.st], g.buf * 8);
+        bulk_copy_g2s(buf, a.rec + line * g.rec, g.rec * 8, &full[at.st]);
+        bulk_copy_g2s(buf + g.rec, a.old + line * g.old, g.old * 8, &full[at.st]);
       }
+      at.next(d, g);
+      ++ahead;
+    } else if (__all_sync(kAllLanes, mbar_look(smem_addr(&empty[done.st]), done.phase))) {
+      write_line<K>(a, bufs + (size_t)done.st * g.buf + g.rec + kOScalars + lane * Ln::kOld,
+                    done.b, done.ch, lane);
+      __syncwarp();  // every lane has read its values before the buffer is filled again
+      done.next(d, g);
+      --ahead;
+      wait = Patience();
+    } else {
+      if (wait.gives_up(a.err, a.timeout_ns)) break;
+      __nanosleep(100);  // leave the issue slots to the solver
     }
-    cp_async_arrive(&full[at.st]);
-    at.next(d.A);
-    ++ahead;
   }
   // After a wait gave up: no copy may still be in flight into this block's
   // memory when it leaves.
-  asm volatile("cp.async.wait_all;" ::: "memory");
   for (; ahead > 0; --ahead) {
     for (int n = 0; n < (1 << 20) && !mbar_test(&full[done.st], done.phase); ++n) {
     }
-    done.next(d.A);
+    done.next(d, g);
   }
 }
 
 // Fetches the lines that the block's first owner needs -- the previous
-// block's last owner's, or the halo -- into the first ring.
+// block's last owner's, or the halo -- into the first ring, as far ahead as
+// it has room, so that the solver never waits for global memory itself.
 template <int K>
 __device__ void fetch_mail(const SweepArgs& a, double* ring, int lane) {
-  using Geo = LineGeo<K>;
+  using Ln = Lanes<K>;
   const Dir& d = a.d;
-  const long long so = d.chain1 ? d.s2 : d.s1;
+  const LineGeo& g = a.g;
   int sl = 0;
-  for (int b = blockIdx.x * Geo::G; b < d.B; b += gridDim.x * Geo::G) {
-    for (int ch = 0; ch < d.A; ++ch) {
+  for (int b = blockIdx.x * g.G; b < d.B; b += gridDim.x * g.G) {
+    double* m = a.mail + (long long)(b / g.G) * d.A * Ln::kMail + lane;
+    for (int ch = 0; ch < d.A; ++ch, m += Ln::kMail) {
       double v[K];
       if (b == 0) {
-        const double* p = a.phi + d.base + ch * d.sa - so;
+        const double* p = a.phi + d.base + ch * d.sa - (d.chain1 ? d.s2 : d.s1);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           const int e = lane * K + k;
           v[k] = e < d.L ? __ldcg(p + e * d.se) : 0.0;
         }
       } else {
-        double* slot = a.mail + ((long long)(b / Geo::G) * d.A + ch) * Geo::W;
-        Patience w;
+        Patience wait;
         for (;;) {
           bool got = true;
 #pragma unroll
-          for (int k = 0; k < K; ++k) {
-            v[k] = ld_relaxed_f64(slot + k * 32 + lane);
-            got = got && !is_empty(v[k]);
-          }
+          for (int k = 0; k < K; ++k) v[k] = ld_relaxed_f64(m + k * 32);
+#pragma unroll
+          for (int k = 0; k < K; ++k) got = got & !is_empty(v[k]);
           if (__all_sync(kAllLanes, got)) break;
-          if (w.gives_up(a.err, a.timeout_ns)) return;
+          if (wait.gives_up(a.err, a.timeout_ns)) return;
         }
 #pragma unroll
-        for (int k = 0; k < K; ++k) st_relaxed_f64(slot + k * 32 + lane, empty_slot());
+        for (int k = 0; k < K; ++k) st_relaxed_f64(m + k * 32, empty_slot());
       }
-      double* to = ring + (size_t)sl * Geo::W;
-      sl = sl + 1 == Geo::kSlots ? 0 : sl + 1;
-      Patience w;
-      for (;;) {
-        bool free = true;
-#pragma unroll
-        for (int k = 0; k < K; ++k) free = free && is_empty(ld_volatile_f64(to + k * 32 + lane));
-        if (__all_sync(kAllLanes, free)) break;
-        if (w.gives_up(a.err, a.timeout_ns)) return;
-      }
-#pragma unroll
-      for (int k = 0; k < K; ++k) st_volatile_f64(to + k * 32 + lane, v[k]);
+      const saddr to = smem_addr(ring + (size_t)sl * g.ring + lane * Ln::kRing);
+      sl = sl + 1 == g.slots ? 0 : sl + 1;
+      Patience wait;
+      while (!__all_sync(kAllLanes, slot_free<K>(to)))
+        if (wait.gives_up(a.err, a.timeout_ns)) return;
+      st_pairs(to, v);
     }
   }
 }
 
 // One lane's segment of the forward recurrence from the entering value, in
 // the sequential operations (division by the stored reciprocal and one
-// correction, which is the correctly rounded quotient: recipdiv.cuh). A
-// segment with an operand outside its range, or a numerator of -0 (the
-// correction would turn it into +0), is redone with `/`; the empty asm keeps
-// that division in a branch of its own (speculated, it doubled a pass).
-template <int K>
+// correction, which is the correctly rounded quotient: recipdiv.cuh). CHECKED,
+// for the pass whose values are kept: a segment with an operand outside the
+// correction's range, or a numerator of -0 (the correction would turn it into
+// +0), is redone with `/`, and its padding elements, which an infinity would
+// reach as 0 * Inf, are cleared. The empty asm keeps that division in a
+// branch of its own (speculated, it doubled a pass).
+template <int K, bool CHECKED>
 __device__ __forceinline__ double forward_segment(const double (&dd)[K], const double (&lo)[K],
                                                   const double (&m)[K], const double (&y)[K],
-                                                  bool y_ok, double in, double (&dp)[K]) {
+                                                  bool y_ok, double in, double (&dp)[K],
+                                                  int elements) {
   bool ok = y_ok;
   double p = in;
 #pragma unroll
@@ -524,16 +663,20 @@ __device__ __forceinline__ double forward_segment(const double (&dd)[K], const d
     const double t = dd[k] - lo[k] * p;
     const double q = t * y[k];
     p = __fma_rn(__fma_rn(-q, m[k], t), y[k], q);
-    ok = ok && (__double_as_longlong(t) == 0 || exp_in_safe_range(t));
+    if (CHECKED) {
+      const int hi = __double2hiint(t);
+      const unsigned e = (unsigned)(hi & 0x7ff00000) - (523u << 20);
+      ok = ok & ((e <= (1000u << 20)) | ((hi | __double2loint(t)) == 0));
+    }
     dp[k] = p;
   }
-  if (!ok) {
+  if (CHECKED && !ok) {
     asm volatile("" ::: "memory");
     p = in;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       p = (dd[k] - lo[k] * p) / m[k];
-      dp[k] = p;
+      dp[k] = k < elements ? p : 0.0;
     }
   }
   return p;
@@ -554,175 +697,227 @@ __device__ __forceinline__ double backward_segment(const double (&dp)[K], const 
 // Passes run before the first look at the fixed point, from the scan steps
 // that the line needs (a measure of its segments' contraction): the scan
 // leaves a few ulps, which two passes absorb where a segment contracts by
-// 2^-7 or more.
+// 2^-7 or more (at most three steps).
 __device__ __forceinline__ int first_passes(int scan_steps) {
-  return scan_steps <= 3 ? 2 : scan_steps;
+  return scan_steps <= 3 ? 2 : scan_steps - 1;
 }
 
+// A line's dependent operations take about 1000 cycles with K = 4 and the
+// instructions around them cost one warp as much again, so everything that
+// can be looked up early is: the next line's hand-over, the state of the slot
+// it goes to and of its buffer are read between this line's two recurrences
+// and settled by a vote beside the vote on the fixed point; only when they
+// were not ready does the warp poll. All 32 lanes take part; those beyond the
+// line read a neutral record (zeros, unit pivots), and their hand-over values
+// are zeros.
+//
+// The lagged coupling of the line's near end, d_1 + a_1 phi_0 (:299-302,
+// :325-328, :352-355), is the recurrence's own step from an entering value
+// phi_0 (d - (-a) phi rounds as d + a phi); the far end's is added to the
+// right-hand side last (-0.0 in the other elements: x + -0.0 is x).
 template <int K, bool CHAIN1>
-__device__ void solve_lines(const SweepArgs& a, int w, double* bufs, uint64_t* full,
-                            uint64_t* empty, double* ring, double* next_ring, int lane) {
-  using Geo = LineGeo<K>;
+__device__ void solve_lines(const SweepArgs& a, int w, saddr bufs, saddr full, saddr empty,
+                            saddr ring, saddr next_ring, saddr neutral, int lane) {
+  using Ln = Lanes<K>;
   const Dir& d = a.d;
+  const LineGeo& g = a.g;
   const long long sc = CHAIN1 ? d.s1 : d.s2;
-  const int last_lane = (d.L - 1) / K;
-  int sl = 0;
-  double x[K];
-  for (LineAt<K> at(w); at.b < d.B; at.next(d.A)) {
-    const bool feeds = at.b + 1 < d.B;
-    const bool in_block = w + 1 < Geo::G;
-    if (at.ch == 0) {  // the chain starts from the halo
-      const double* p = a.phi + d.base + at.b * d.sb - sc;
+  const bool on = lane < g.n;
+  const bool first = lane == 0 || !on, last = lane >= g.n - 1;
+  const bool near_end = lane == 0 && d.L > 1;
+  const bool in_block = w + 1 < g.G;
+  const int elements = d.L - lane * K;  // this lane's, if less than K
+  const saddr buf_bytes = 8u * g.buf, bufs_end = bufs + g.NB * buf_bytes;
+  const saddr slot_bytes = 8u * g.ring, slots_bytes = g.slots * slot_bytes;
+  const saddr rec_at = 8u * (kRScalars + lane * Ln::kRec);
+  const saddr old_at = 8u * (g.rec + kOScalars + lane * Ln::kOld);
+  ring += 8u * lane * Ln::kRing;
+  next_ring += 8u * lane * Ln::kRing;
+  saddr buf = bufs, bar = 0, slot = 0;  // this line's buffer, barriers and slots
+  uint32_t phase = 0;
+  double x[K], t2[K];
+  bool go = false;  // the hand-over, its target slot and the buffer are ready
+  for (int b = blockIdx.x * g.G + w; b < d.B; b += gridDim.x * g.G) {
+    const bool feeds = b + 1 < d.B;
+    double* mail =
+        a.mail + (long long)((b + 1) / g.G) * d.A * Ln::kMail + lane;  // of the next block
+    {  // the chain starts from the halo
+      const double* p = a.phi + d.base + b * d.sb - sc;
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const int e = lane * K + k;
         x[k] = e < d.L ? __ldcg(p + e * d.se) : 0.0;
       }
     }
-    const bool here = mbar_wait(&full[at.st], at.phase, a.err, a.timeout_ns);
-    if (!__all_sync(kAllLanes, here)) return;
-    double* buf = bufs + (size_t)at.st * Geo::kBuf;
-    auto op = [buf, lane](int arr, int k) { return buf[arr * Geo::W + k * 32 + lane]; };
-    double lo[K], m[K], y[K], cp[K], dd[K], t2[K];
-    bool y_ok = true;
+    for (int ch = 0; ch < d.A; ++ch) {
+      if (!go) {
+        Patience wait;
+        for (;;) {
+          bool ready = slot_full<K>(ring + slot, t2);
+          if (feeds && in_block) ready = ready & slot_free<K>(next_ring + slot);
+          ready = ready & mbar_look(full + bar, phase);
+          if (__all_sync(kAllLanes, ready)) break;
+          if (wait.gives_up(a.err, a.timeout_ns)) return;
+        }
+      }
+      const saddr r = on ? buf + rec_at : neutral;
+      const saddr old = on ? buf + old_at : neutral + 8u * Ln::kRec;
+      // Right-hand side, in the reference's order.
+      double dd[K], lo[K], m[K], y[K], cp[K], scan[2 * kScanSteps], scalars[kRScalars], ends[2];
+      {
+        double su[K], c1m[K], c2m[K], ov[kOArrays * K];
+        ld_pairs(r + 8 * kRSu * K, su);
+        ld_pairs(r + 8 * kR1m * K, c1m);
+        ld_pairs(old, ov);
+        ld_pairs(r + 8 * kR2m * K, c2m);
+        ld_pairs(r + 8 * kRLo * K, lo);
+        ld_pairs(r + 8 * kRY * K, y);
+        ld_pairs(buf, scalars);
+        ld_pairs(buf + 8 * g.rec, ends);
+        ld_pairs(r + 8 * Ln::kScan, scan);
+        ld_pairs(r + 8 * kRM * K, m);
+        ld_pairs(r + 8 * kRCp * K, cp);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      lo[k] = op(kRLo, k);
-      m[k] = op(kRM, k);
-      y[k] = op(kRY, k);
-      cp[k] = op(kRCp, k);
-      y_ok = y_ok && y[k] != 0.0;
-    }
-    const double end0 = buf[Geo::kScalars + kRE0] * buf[Geo::kEnds];
-    const double end1 = buf[Geo::kScalars + kRE1] * buf[Geo::kEnds + 1];
-    const int nf = (int)buf[Geo::kScalars + kRNf], nb = (int)buf[Geo::kScalars + kRNb];
-    double sf[kScanSteps], sb[kScanSteps];
+        for (int k = 0; k < K; ++k) {
+          const double n1 = CHAIN1 ? x[k] : t2[k], n2 = CHAIN1 ? t2[k] : x[k];
+          double t = su[k] + c1m[k] * n1;
+          t = t + ov[kO1 * K + k];
+          t = t + c2m[k] * n2;
+          t = t + ov[kO2 * K + k];
+          dd[k] = t + ov[kOEnd * K + k];
+        }
+      }
+      if (d.L == 1 && lane == 0)  // both ends in one element
+        dd[0] = (dd[0] + scalars[kRE0] * ends[0]) + scalars[kRE1] * ends[1];
 #pragma unroll
-    for (int s = 0; s < kScanSteps; ++s) {
-      sf[s] = buf[Geo::kScanF + 32 * s + lane];
-      sb[s] = buf[Geo::kScanB + 32 * s + lane];
-    }
-    double* to = next_ring + (size_t)sl * Geo::W;
-    if (!take_slot<K>(a, ring + (size_t)sl * Geo::W, feeds && in_block ? to : nullptr, lane, t2))
-      return;
-    sl = sl + 1 == Geo::kSlots ? 0 : sl + 1;
-    // right-hand side, the reference's order; the lagged couplings of the
-    // segment ends come last (:299-302, :325-328, :352-355)
+      for (int k = 0; k < K; k += 2) st_pair(ring + slot + 8 * k, empty_slot(), empty_slot());
+      // Forward: entering values from the scan, then the passes.
+      const int nfu = (int)scalars[kRNf], nf = nfu & (kUnsafe - 1), nb = (int)scalars[kRNb];
+      const bool y_ok = nfu < kUnsafe;
+      const double enter = near_end ? ends[0] : 0.0;
+      double dp[K];
+      double u = enter;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int e = lane * K + k;
-      const double n1 = CHAIN1 ? x[k] : t2[k], n2 = CHAIN1 ? t2[k] : x[k];
-      double t = op(kRSu, k) + op(kR1m, k) * n1;
-      t = t + op(kR1p, k) * buf[Geo::kP1 + k * 32 + lane];
-      t = t + op(kR2m, k) * n2;
-      t = t + op(kR2p, k) * buf[Geo::kP2 + k * 32 + lane];
-      if (e == 0) t = t + end0;
-      if (e == d.L - 1) t = t + end1;
-      dd[k] = t;
-    }
-    // Forward: entering values from the scan, then the passes.
-    double dp[K];
-    double u = 0.0;
+      for (int k = 0; k < K; ++k) u = __fma_rn(-lo[k] * y[k], u, dd[k] * y[k]);
+      constexpr int kFew = 3;  // steps taken without a look at the count
 #pragma unroll
-    for (int k = 0; k < K; ++k) u = __fma_rn(-lo[k] * y[k], u, dd[k] * y[k]);
+      for (int s = 0; s < kFew; ++s)
+        u = __fma_rn(scan[2 * s], __shfl_up_sync(kAllLanes, u, 1 << s), u);
+      if (nf > kFew) {
 #pragma unroll
-    for (int s = 0; s < kScanSteps; ++s)
-      if (s < nf) u = __fma_rn(sf[s], __shfl_up_sync(kAllLanes, u, 1 << s), u);
-    auto enter_f = [lane](double out) {
-      const double v = __shfl_up_sync(kAllLanes, out, 1);
-      return lane == 0 ? 0.0 : v;
-    };
-    double inf = enter_f(u), nin = inf;
-    for (int n = first_passes(nf); n > 0; --n) {
+        for (int s = kFew; s < kScanSteps; ++s)
+          u = __fma_rn(scan[2 * s], __shfl_up_sync(kAllLanes, u, 1 << s), u);
+      }
+      auto enter_f = [first, enter](double out) {
+        const double v = __shfl_up_sync(kAllLanes, out, 1);
+        return first ? enter : v;
+      };
+      auto forward = [&](double in) {
+        return enter_f(forward_segment<K, true>(dd, lo, m, y, y_ok, in, dp, elements));
+      };
+      double inf = enter_f(u);
+      inf = enter_f(forward_segment<K, false>(dd, lo, m, y, y_ok, inf, dp, elements));
+      for (int n = first_passes(nf); n > 2; --n)
+        inf = enter_f(forward_segment<K, false>(dd, lo, m, y, y_ok, inf, dp, elements));
+      double nin = forward(inf);
+      bool settled = same_bits(nin, inf);
       inf = nin;
-      nin = enter_f(forward_segment<K>(dd, lo, m, y, y_ok, inf, dp));
-    }
-    bool settled = same_bits(nin, inf);
-    inf = nin;
-    // Backward, likewise; padding elements enter it as zeros whatever the
-    // forward passes left in them (0 * Inf), so the last element is dp itself.
-    auto clear_pads = [&] {
+      // A first look at what the next line needs.
+      const saddr this_to = next_ring + slot, this_old = old, this_empty = empty + bar;
+      slot = slot + slot_bytes == slots_bytes ? 0 : slot + slot_bytes;
+      buf += buf_bytes;
+      bar += 8;
+      if (buf == bufs_end) {
+        buf = bufs;
+        bar = 0;
+        phase ^= 1u;
+      }
+      bool ready = slot_full<K>(ring + slot, t2);
+      if (in_block) ready = ready & slot_free<K>(next_ring + slot);
+      ready = ready & mbar_look(full + bar, phase);
+      // Backward, likewise.
+      u = 0.0;
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (lane * K + k >= d.L) dp[k] = 0.0;
-    };
-    clear_pads();
-    u = 0.0;
+      for (int k = K - 1; k >= 0; --k) u = __fma_rn(-cp[k], u, dp[k]);
 #pragma unroll
-    for (int k = K - 1; k >= 0; --k) u = __fma_rn(-cp[k], u, dp[k]);
+      for (int s = 0; s < kFew; ++s)
+        u = __fma_rn(scan[2 * s + 1], __shfl_down_sync(kAllLanes, u, 1 << s), u);
+      if (nb > kFew) {
 #pragma unroll
-    for (int s = 0; s < kScanSteps; ++s)
-      if (s < nb) u = __fma_rn(sb[s], __shfl_down_sync(kAllLanes, u, 1 << s), u);
-    auto enter_b = [lane, last_lane](double out) {
-      const double v = __shfl_down_sync(kAllLanes, out, 1);
-      return lane >= last_lane ? 0.0 : v;
-    };
-    double inb = enter_b(u);
-    nin = inb;
-    for (int n = first_passes(nb); n > 0; --n) {
-      inb = nin;
+        for (int s = kFew; s < kScanSteps; ++s)
+          u = __fma_rn(scan[2 * s + 1], __shfl_down_sync(kAllLanes, u, 1 << s), u);
+      }
+      auto enter_b = [last](double out) {
+        const double v = __shfl_down_sync(kAllLanes, out, 1);
+        return last ? 0.0 : v;
+      };
+      double inb = enter_b(u);
+      inb = enter_b(backward_segment<K>(dp, cp, inb, x));
+      for (int n = first_passes(nb); n > 2; --n)
+        inb = enter_b(backward_segment<K>(dp, cp, inb, x));
       nin = enter_b(backward_segment<K>(dp, cp, inb, x));
-    }
-    settled = settled && same_bits(nin, inb);
-    inb = nin;
-    if (!__all_sync(kAllLanes, settled)) {  // on to the fixed points, each at most 32 passes away
-      for (int n = 0; n <= 32; ++n) {
-        nin = enter_f(forward_segment<K>(dd, lo, m, y, y_ok, inf, dp));
-        if (__all_sync(kAllLanes, same_bits(nin, inf))) break;
-        inf = nin;
+      settled = settled & same_bits(nin, inb);
+      inb = nin;
+      go = __all_sync(kAllLanes, ready);
+      if (!__all_sync(kAllLanes, settled)) {  // on to the fixed points, at most 32 passes away
+        for (int n = 0; n <= 32; ++n) {
+          nin = forward(inf);
+          if (__all_sync(kAllLanes, same_bits(nin, inf))) break;
+          inf = nin;
+        }
+        for (int n = 0; n <= 32; ++n) {
+          nin = enter_b(backward_segment<K>(dp, cp, inb, x));
+          if (__all_sync(kAllLanes, same_bits(nin, inb))) break;
+          inb = nin;
+        }
       }
-      clear_pads();
-      for (int n = 0; n <= 32; ++n) {
-        nin = enter_b(backward_segment<K>(dp, cp, inb, x));
-        if (__all_sync(kAllLanes, same_bits(nin, inb))) break;
-        inb = nin;
+      if (feeds && in_block) {
+        st_pairs(this_to, x);
+      } else if (feeds) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) st_relaxed_f64(mail + k * 32, x[k]);
+        mail += Ln::kMail;
       }
+      if (on) st_pairs(this_old, x);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(this_empty);
     }
-    if (feeds && in_block) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) st_volatile_f64(to + k * 32 + lane, x[k]);
-    } else if (feeds) {
-      double* mail = a.mail + ((long long)((at.b + 1) / Geo::G) * d.A + at.ch) * Geo::W;
-#pragma unroll
-      for (int k = 0; k < K; ++k) st_relaxed_f64(mail + k * 32 + lane, x[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) buf[Geo::kP1 + k * 32 + lane] = x[k];
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[at.st]);
   }
 }
 
-// Warps 0..G-1 solve, G..2G-1 load and write, 2G fetches the mail. A warp whose wait
-// gave up leaves; the others' waits see the error word and leave too.
+// Warps 0..G-1 solve, G..2G-1 load and write, 2G fetches the mail. A warp
+// whose wait gave up leaves; the others' waits see the error word and leave
+// too.
 template <int K, bool CHAIN1>
-__global__ void __launch_bounds__(LineGeo<K>::kThreads, 1) tdma_sweep_kernel(SweepArgs a) {
-  using Geo = LineGeo<K>;
+__global__ void __launch_bounds__(Lanes<K>::kMaxThreads, 1) tdma_sweep_kernel(SweepArgs a) {
+  using Ln = Lanes<K>;
   extern __shared__ __align__(128) double sm[];
-  __shared__ __align__(8) uint64_t full[Geo::G][Geo::NB], empty[Geo::G][Geo::NB];
+  __shared__ __align__(8) uint64_t full[Ln::kMaxOwners][4], empty[Ln::kMaxOwners][4];
+  const LineGeo& g = a.g;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double* rings = sm + (size_t)Geo::G * Geo::NB * Geo::kBuf;
-  for (int i = threadIdx.x; i < Geo::G * Geo::kSlots * Geo::W; i += Geo::kThreads)
-    rings[i] = empty_slot();
-  // padding elements' neighbour values are never loaded
-  for (int i = threadIdx.x; i < Geo::G * Geo::NB * 2 * Geo::W; i += Geo::kThreads)
-    sm[(size_t)(i / (2 * Geo::W)) * Geo::kBuf + Geo::kP1 + i % (2 * Geo::W)] = 0.0;
+  double* rings = sm + (size_t)g.G * g.NB * g.buf;
+  const int ring = g.slots * g.ring;
+  double* neutral = rings + g.G * ring;
+  for (int i = threadIdx.x; i < g.G * ring; i += blockDim.x) rings[i] = empty_slot();
+  for (int i = threadIdx.x; i < Ln::kRec + Ln::kOld; i += blockDim.x)
+    neutral[i] = i >= kRM * K && i < (kRY + 1) * K ? 1.0 : 0.0;
   if (threadIdx.x == 0) {
-    for (int g = 0; g < Geo::G; ++g)
-      for (int n = 0; n < Geo::NB; ++n) {
-        mbar_init(&full[g][n], 33);  // the bulk copy's expect and 32 lanes' copies
-        mbar_init(&empty[g][n], 1);
+    for (int o = 0; o < g.G; ++o)
+      for (int n = 0; n < g.NB; ++n) {
+        mbar_init(&full[o][n], 1);
+        mbar_init(&empty[o][n], 1);
       }
     mbar_fence_init();
   }
   __syncthreads();
-  if (warp < Geo::G) {
-    solve_lines<K, CHAIN1>(a, warp, sm + (size_t)warp * Geo::NB * Geo::kBuf, full[warp],
-                           empty[warp], rings + (size_t)warp * Geo::kSlots * Geo::W,
-                           rings + (size_t)(warp + 1) * Geo::kSlots * Geo::W, lane);
-  } else if (warp < 2 * Geo::G) {
-    const int w = warp - Geo::G;
-    load_lines<K>(a, w, sm + (size_t)w * Geo::NB * Geo::kBuf, full[w], empty[w], lane);
+  if (warp < g.G) {
+    solve_lines<K, CHAIN1>(a, warp, smem_addr(sm + (size_t)warp * g.NB * g.buf),
+                           smem_addr(full[warp]), smem_addr(empty[warp]),
+                           smem_addr(rings + (size_t)warp * ring),
+                           smem_addr(rings + (size_t)(warp + 1) * ring), smem_addr(neutral), lane);
+  } else if (warp < 2 * g.G) {
+    const int w = warp - g.G;
+    load_lines<K>(a, w, sm + (size_t)w * g.NB * g.buf, full[w], empty[w], lane);
   } else {
     fetch_mail<K>(a, rings, lane);
   }
@@ -856,22 +1051,18 @@ __global__ void div_check_kernel(long long n, unsigned long long seed,
   atomicAdd(counts + 1, fast);
 }
 
-// Elements per lane of a line of L: the next instantiated size.
+// Elements per lane of a line of L: four (see the file comment), beyond 128
+// the next instantiated size.
 int line_k(int L) {
   const int k = (L + 31) / 32;
-  return k <= 8 ? k : k <= 12 ? 12 : k <= 16 ? 16 : k <= 24 ? 24 : 32;
+  return k <= 4 ? 4 : k <= 6 ? 6 : k <= 8 ? 8 : k <= 12 ? 12 : k <= 16 ? 16 : k <= 24 ? 24 : 32;
 }
 
 template <class F>
-auto with_k(int k, F f) {
-  switch (k) {
-    case 1: return f(std::integral_constant<int, 1>());
-    case 2: return f(std::integral_constant<int, 2>());
-    case 3: return f(std::integral_constant<int, 3>());
+auto with_k(int L, F f) {
+  switch (line_k(L)) {
     case 4: return f(std::integral_constant<int, 4>());
-    case 5: return f(std::integral_constant<int, 5>());
     case 6: return f(std::integral_constant<int, 6>());
-    case 7: return f(std::integral_constant<int, 7>());
     case 8: return f(std::integral_constant<int, 8>());
     case 12: return f(std::integral_constant<int, 12>());
     case 16: return f(std::integral_constant<int, 16>());
@@ -921,32 +1112,53 @@ Dir make_dir(const HaloInputs& in, int nr, int nth, int nz, int dir) {
 }
 
 struct DirSizes {
-  size_t rec, mail;  // doubles
+  size_t rec, old, mail;  // doubles
   int blocks, threads;
 };
 
 DirSizes dir_sizes(const Dir& d) {
-  return with_k(line_k(d.L), [&d](auto k) {
-    using Geo = LineGeo<decltype(k)::value>;
-    const int blocks = (d.B + Geo::G - 1) / Geo::G;
-    return DirSizes{(size_t)d.A * d.B * Geo::kRec, (size_t)blocks * d.A * Geo::W, blocks,
-                    Geo::kThreads};
+  return with_k(d.L, [&d](auto k) {
+    constexpr int K = decltype(k)::value;
+    const LineGeo g = line_geo<K>(d.L);
+    const int blocks = (d.B + g.G - 1) / g.G;
+    return DirSizes{(size_t)d.A * d.B * g.rec, (size_t)d.A * d.B * g.old, (size_t)blocks * d.A * Lanes<K>::kMail, blocks,
+                    32 * (2 * g.G + 1)};
   });
 }
 
-template <int K, bool CHAIN1>
-cudaError_t launch_sweep(const SweepArgs& a, int sms, cudaStream_t st) {
-  using Geo = LineGeo<K>;
-  const void* k = (const void*)tdma_sweep_kernel<K, CHAIN1>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)Geo::kSmem);
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  return bytes <= 48 * 1024
+             ? cudaSuccess
+             : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)bytes);
+}
+
+// Launches a kernel over tiles of lines whose records of `rec` doubles are
+// built in shared memory: eight lines a block (64-byte rows, a warp a line),
+// fewer where three blocks' records would not fit an SM.
+template <class Args>
+cudaError_t launch_tiles(void (*kernel)(Args), Args a, int rec, cudaStream_t st) {
+  const size_t bytes = (size_t)rec * sizeof(double);
+  a.tile = 8;
+  while (a.tile > 1 && a.tile * bytes > 75 * 1024) a.tile /= 2;
+  const int U = a.d.b_fast ? a.d.B : a.d.A, V = a.d.b_fast ? a.d.A : a.d.B;
+  const long long grid = (long long)((U + a.tile - 1) / a.tile) * V;
+  const cudaError_t e = allow_smem((const void*)kernel, a.tile * bytes);
   if (e != cudaSuccess) return e;
-  // One block per SM; further owners follow in rounds.
-  const int blocks = (a.d.B + Geo::G - 1) / Geo::G;
-  SweepArgs copy = a;
-  void* args[] = {&copy};
-  return cudaLaunchCooperativeKernel(k, dim3(blocks < sms ? blocks : sms), dim3(Geo::kThreads),
-                                     args, Geo::kSmem, st);
+  kernel<<<(unsigned)grid, kTileBlock, a.tile * bytes, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int K, bool CHAIN1>
+cudaError_t launch_sweep(SweepArgs a, int sms, cudaStream_t st) {
+  const void* k = (const void*)tdma_sweep_kernel<K, CHAIN1>;
+  const cudaError_t e = allow_smem(k, a.g.smem);
+  if (e != cudaSuccess) return e;
+  // At most one block per SM; further owners follow in rounds.
+  const int blocks = (a.d.B + a.g.G - 1) / a.g.G;
+  void* args[] = {&a};
+  return cudaLaunchCooperativeKernel(k, dim3(blocks < sms ? blocks : sms),
+                                     dim3(32 * (2 * a.g.G + 1)), args, a.g.smem, st);
 }
 
 }  // namespace
@@ -961,10 +1173,13 @@ size_t tdma_mailbox_doubles(int nr, int nth, int nz) {
 }
 
 size_t tdma_factor_doubles(int nr, int nth, int nz) {
-  size_t sum = 0;
-  for (int dir = 0; dir < 3; ++dir)
-    sum += dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir)).rec;
-  return sum;
+  size_t sum = 0, old = 0;
+  for (int dir = 0; dir < 3; ++dir) {
+    const DirSizes s = dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir));
+    sum += s.rec;
+    if (s.old > old) old = s.old;
+  }
+  return sum + old;  // every direction's records, one direction's old values
 }
 
 void tdma_launch_shape(int nr, int nth, int nz, int sms, int* grid, int* block) {
@@ -998,28 +1213,34 @@ cudaError_t launch_tdma_f64(const HaloInputs& in, double* phi, int nr, int nth, 
     f.nz = nz;
     rec[dir] = fac;
     fac += dir_sizes(f.d).rec;
-    const long long lines = (long long)f.d.A * f.d.B;
-    long long grid = (lines + kFactorBlock / 32 - 1) / (kFactorBlock / 32);
-    if (grid > 8LL * sms) grid = 8LL * sms;
-    with_k(line_k(f.d.L), [&](auto k) {
-      tdma_factor_kernel<decltype(k)::value><<<(unsigned)grid, kFactorBlock, 0, st>>>(f);
-      return 0;
+    const cudaError_t e = with_k(f.d.L, [&](auto k) {
+      constexpr int K = decltype(k)::value;
+      f.g = line_geo<K>(f.d.L);
+      return launch_tiles(tdma_factor_kernel<K>, f, f.g.rec, st);
     });
-    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
+  double* const old = fac;
   for (int sweep = 1; sweep <= n_sweep; ++sweep) {
     for (int dir = 0; dir < 3; ++dir) {
+      OldArgs o;
+      o.d = make_dir(in, nr, nth, nz, dir);
+      o.phi = phi;
+      o.old = old;
       SweepArgs a;
-      a.d = make_dir(in, nr, nth, nz, dir);
+      a.d = o.d;
       if (dir == 2 && sweep == n_sweep) a.d.wrap = 0;  // no refresh after the last direction
       a.rec = rec[dir];
+      a.old = old;
       a.mail = mbox;
       a.phi = phi;
       a.err = ws.err;
       a.timeout_ns = timeout_ns;
-      const cudaError_t e = with_k(line_k(a.d.L), [&](auto k) {
+      const cudaError_t e = with_k(a.d.L, [&](auto k) {
         constexpr int K = decltype(k)::value;
+        o.g = a.g = line_geo<K>(a.d.L);
+        const cudaError_t e2 = launch_tiles(tdma_old_kernel<K>, o, o.g.old, st);
+        if (e2 != cudaSuccess) return e2;
         return a.d.chain1 ? launch_sweep<K, true>(a, sms, st) : launch_sweep<K, false>(a, sms, st);
       });
       if (e != cudaSuccess) return e;
