@@ -58,25 +58,14 @@ int finish_tdma(eaf_cg* h, bool host_path, int n_sweep) {
   return err;
 }
 
-int residual_launch_shape(const eaf_cg* h, int* grid, int* block) {
-  const int b = 512;
-  long long g = ((long long)h->d.n + 4095) / 4096;
-  if (g < 1) g = 1;
-  if (g > h->sms) g = h->sms;
-  *grid = (int)g;
-  *block = b;
-  return EAF_OK;
-}
-
 int run_residual(eaf_cg* h, const HaloInputs& in, const double* phi, double* residual) {
   int grid, block;
-  residual_launch_shape(h, &grid, &block);
+  eaf::residual_launch_shape(h->d.n, h->sms, &grid, &block);
   h->last_grid = grid;
   h->last_block = block;
   h->last_cluster = 1;
   EAF_CUDA(cudaEventRecord(h->ev[2], h->st));
-  EAF_CUDA(eaf::launch_residual_f64(in, phi, h->d, h->ws, h->timeout_ns, grid, block,
-                                    h->st));
+  EAF_CUDA(eaf::launch_residual_f64(in, phi, h->d, h->ws, h->timeout_ns, grid, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(cudaMemcpyAsync(h->res_h, h->ws.result, sizeof(SolveResult),
                            cudaMemcpyDeviceToHost, h->st));

@@ -230,11 +230,12 @@ void tdma_launch_shape(int nr, int nth, int nz, int sms, int* grid, int* block);
 cudaError_t launch_tdma_f64(const HaloInputs& in, double* phi, int nr, int nth, int nz,
                             int n_sweep, double* mbox, double* fac, int sms, const GroupWs& ws,
                             uint64_t timeout_ns, cudaStream_t st);
-// compute_residual_3d_mpi (serial) into ws.result->residual.
+// compute_residual_3d_mpi (serial) into ws.result->residual, on the grid that
+// residual_launch_shape gives for n cells.
+void residual_launch_shape(long long n, int sms, int* grid, int* block);
 cudaError_t launch_residual_f64(const HaloInputs& in, const double* phi, const MeshDims& d,
-                                const GroupWs& ws, uint64_t timeout_ns, int grid, int block,
+                                const GroupWs& ws, uint64_t timeout_ns, int grid,
                                 cudaStream_t st);
-const void* residual_kernel_ptr();
 // Counts[0] = pairs where the TDMA's reciprocal-corrected division differs
 // from `/` in any bit, counts[1] = pairs that took its fast path.
 cudaError_t run_div_check(long long n, unsigned long long seed, unsigned long long* counts,

@@ -937,7 +937,13 @@ struct ResArgs {
   uint64_t timeout_ns;
 };
 
-__global__ void __launch_bounds__(1024) residual_kernel(ResArgs a) {
+// Bound by memory: every load of a cell (the identity-row test needs the
+// coefficients, the residual also seven values of phi) is issued before the
+// first decision, and 64 registers a thread leave room for two blocks of 512
+// on an SM.
+constexpr int kResBlock = 512;
+
+__global__ void __launch_bounds__(kResBlock, 2) residual_kernel(ResArgs a) {
   Group g;
   g.counter = a.ws.counter;
   g.err = a.ws.err;
@@ -950,26 +956,24 @@ __global__ void __launch_bounds__(1024) residual_kernel(ResArgs a) {
   const Slice own = own_slice(a.d.n, g.nb, g.bid);
   double v[2] = {0.0, 0.0};
   const HaloInputs& in = a.in;
-  for (int c = own.begin + (int)threadIdx.x; c < own.end; c += blockDim.x) {
+  const double* __restrict__ ph = a.phi;
+  for (int c = own.begin + (int)threadIdx.x; c < own.end; c += kResBlock) {
     int i, j, k;
     cell_ijk(a.d, c, i, j, k);
     const long long q = (i + 2) + a.sx * (j + 2) + a.sxy * (k + 2);
-    const double P = in.aP[q], W = in.aW[q], E = in.aE[q], S = in.aS[q], N = in.aN[q],
-                 B = in.aB[q], T = in.aT[q], U = in.Su[q];
-    if (P == 1.0 && W == 0.0 && E == 0.0 && S == 0.0 && N == 0.0 && B == 0.0 &&
-        T == 0.0) {
-      v[0] = v[0] + 0.0;
-      v[1] = v[1] + 0.0;
-      continue;
-    }
-    const double* ph = a.phi;
-    const double pc = ph[q];
-    double r = U - P * pc + S * ph[q - a.sx] + N * ph[q + a.sx];
-    r = r + W * ph[q - 1] + E * ph[q + 1];
-    r = r + B * ph[q - a.sxy] + T * ph[q + a.sxy];
+    const double P = __ldg(in.aP + q), W = __ldg(in.aW + q), E = __ldg(in.aE + q),
+                 S = __ldg(in.aS + q), N = __ldg(in.aN + q), B = __ldg(in.aB + q),
+                 T = __ldg(in.aT + q), U = __ldg(in.Su + q);
+    const double pc = ph[q], pw = ph[q - 1], pe = ph[q + 1], ps = ph[q - a.sx],
+                 pn = ph[q + a.sx], pb = ph[q - a.sxy], pt = ph[q + a.sxy];
+    const bool trivial = (P == 1.0) & (W == 0.0) & (E == 0.0) & (S == 0.0) & (N == 0.0) &
+                         (B == 0.0) & (T == 0.0);
+    double r = U - P * pc + S * ps + N * pn;
+    r = r + W * pw + E * pe;
+    r = r + B * pb + T * pt;
     const double t = fabs(U) + fabs(P * pc) + kSmall;
-    v[0] = v[0] + r * r;
-    v[1] = v[1] + t * t;
+    v[0] = v[0] + (trivial ? 0.0 : r * r);
+    v[1] = v[1] + (trivial ? 0.0 : t * t);
   }
   const bool ok = group_allsum<2>(v, g, 0);
   if (g.bid == 0 && threadIdx.x == 0) {
@@ -1249,8 +1253,15 @@ cudaError_t launch_tdma_f64(const HaloInputs& in, double* phi, int nr, int nth, 
   return cudaSuccess;
 }
 
+// A cell a thread up to two blocks per SM (more cells in turn beyond).
+void residual_launch_shape(long long n, int sms, int* grid, int* block) {
+  const long long g = (n + kResBlock - 1) / kResBlock;
+  *grid = (int)(g < 2 * sms ? g : 2 * sms);
+  *block = kResBlock;
+}
+
 cudaError_t launch_residual_f64(const HaloInputs& in, const double* phi, const MeshDims& d,
-                                const GroupWs& ws, uint64_t timeout_ns, int grid, int block,
+                                const GroupWs& ws, uint64_t timeout_ns, int grid,
                                 cudaStream_t st) {
   ResArgs a;
   a.in = in;
@@ -1264,11 +1275,10 @@ cudaError_t launch_residual_f64(const HaloInputs& in, const double* phi, const M
   if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
-  return cudaLaunchCooperativeKernel((const void*)residual_kernel, dim3(grid), dim3(block),
+  return cudaLaunchCooperativeKernel((const void*)residual_kernel, dim3(grid), dim3(kResBlock),
                                      args, 0, st);
 }
 
-const void* residual_kernel_ptr() { return (const void*)residual_kernel; }
 
 cudaError_t run_div_check(long long n, unsigned long long seed, unsigned long long* counts,
                           cudaStream_t st) {
