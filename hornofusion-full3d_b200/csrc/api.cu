@@ -99,6 +99,11 @@ static int max_coresident(const void* kernel, int block, int sms) {
 
 namespace eaf {
 
+// Kept operands pay while they leave the SM's L1 some room: 190 KB a block
+// 15.0 against 16.9 us per iteration (878,560 cells), 224 KB 21.2 against 19.6
+// (1,036,800 cells).
+constexpr size_t kKeepPays = 200 * 1024;
+
 std::mutex& launch_attr_mutex() {
   static std::mutex m;
   return m;
@@ -106,8 +111,9 @@ std::mutex& launch_attr_mutex() {
 
 // Launch shape for a persistent kernel over n cells: an explicit
 // eaf_cg_set_launch shape, else the tuned shape of this mesh (FP64 solver),
-// else, for the reference-form FP64 solver on a mesh that fits, one
-// cluster-resident launch (below), else one 1024-thread block up to 8192
+// else, for the reference-form FP64 solver, one cluster-resident launch where
+// the mesh fits one and a 512-thread block on every SM beyond (below), else
+// (other forms, a requested cluster size) one 1024-thread block up to 8192
 // cells or one 512-thread block per 2048 cells; capped by co-residency of
 // the kernel (variant) that runs blocks of that size. The reference-form FP64 solver may run on a grid of
 // thread-block clusters (eaf_cg_set_cluster, else the tuned cluster size):
@@ -138,6 +144,7 @@ SolverLaunch choose_launch(int nr, int nth, int nz, int sms, int req_block, int 
     g = (int)(want < 1 ? 1 : want);
   }
   int c = 1;
+  bool spread = false;
   if (automatic && f64 && form == EAF_CG_FORM_REFERENCE && !tuned && req_cluster == 0) {
     // A small mesh outside the table: one cluster that keeps the system in
     // its shared memory (8 blocks up to 8192 cells, else 16), one cell per
@@ -151,6 +158,15 @@ SolverLaunch choose_launch(int nr, int nth, int nz, int sms, int req_block, int 
       b = bs;
       g = cs;
       tc = cs;
+    } else if (n > 8192) {
+      // Beyond a cluster: every SM, 512 threads a block, the own cells' update
+      // operands kept in shared memory. Against 512 threads per 2048 cells
+      // and per-thread loads, us per iteration: 31,680 cells 6.4 / 8.0, 78,408
+      // 6.5 / 8.4, 121,296 6.9 / 8.3, 193,971 7.9 / 8.4, 389,376 10.3 / 10.9,
+      // 878,560 15.0 / 16.9; blocks of 256 or 1024 threads were slower from
+      // 120,000 cells on and within 2 % below.
+      g = sms < 32 * kPerLane ? sms : 32 * kPerLane;
+      spread = true;
     }
   }
   if (f64 && form == EAF_CG_FORM_REFERENCE) {
@@ -176,7 +192,8 @@ SolverLaunch choose_launch(int nr, int nth, int nz, int sms, int req_block, int 
       k = !automatic ? EAF_CG_KERNEL_LOADS
           : ts == 2  ? EAF_CG_KERNEL_KEEP
           : ts == 1  ? EAF_CG_KERNEL_STREAM
-                     : EAF_CG_KERNEL_LOADS;
+          : spread && keep_smem_bytes(n, g) <= kKeepPays ? EAF_CG_KERNEL_KEEP
+                                                         : EAF_CG_KERNEL_LOADS;
     slots = k == EAF_CG_KERNEL_SLOTS;
     stream = k == EAF_CG_KERNEL_STREAM;
     keep = k == EAF_CG_KERNEL_KEEP;

@@ -46,14 +46,12 @@ constexpr int kNoallocMaxCells = EAF_NOALLOC_MAX_CELLS;
 // for it. Every launch shape the handle entries pick for a mesh of at most
 // kNoallocMaxCells cells must fit, or the two would not give the same bits:
 // the tuned shapes (checked here), the small-mesh fallback of one cluster
-// of at most 16 blocks, and the fallback without clusters of one 512-thread
-// block per 2048 cells (checked here).
-constexpr int kNoallocMaxBlocks = 64;
+// of at most 16 blocks, and the fallback of one block per SM, at most as many
+// as the slot all-reduce reads.
+constexpr int kNoallocMaxBlocks = 32 * eaf::kPerLane;
 static_assert(eaf::max_tuned_grid_up_to(kNoallocMaxCells) <= kNoallocMaxBlocks,
               "a tuned launch for a mesh within the no-allocation limit has more "
               "blocks than the static scratch holds partials for");
-static_assert((kNoallocMaxCells + 2047) / 2048 <= kNoallocMaxBlocks,
-              "the fallback launch shape exceeds the static scratch's block limit");
 constexpr int kPartSlots = 8;
 // A cluster launch uses the partial table as its slot table: at most
 // kNoallocMaxBlocks / 2 clusters of two or more blocks.
@@ -172,7 +170,7 @@ extern "C" int eaf_cg_solve_f64_noalloc(int nr, int nth, int nz, int device,
   }
   const eaf::SolverLaunch L =
       eaf::choose_launch(nr, nth, nz, sms, 0, 0, 0, EAF_CG_FORM_REFERENCE, true);
-  if (L.grid > kNoallocMaxBlocks) {  // excluded by the static_asserts above
+  if (L.grid > kNoallocMaxBlocks) {  // excluded by the static_assert above
     eaf::set_error_text("eaf_cg_solve_f64_noalloc: launch shape exceeds the static scratch");
     return EAF_EINVAL;
   }
