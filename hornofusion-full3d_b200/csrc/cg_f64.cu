@@ -91,6 +91,7 @@ struct CgArgs {
   int max_iter;
   double tol;
   uint64_t timeout_ns;
+  int keep_r = 0;  // PF: own cells whose residual stays in shared memory
 };
 
 // Loops over this thread's cells of the block slice in rounds of U cells
@@ -101,9 +102,15 @@ struct CgArgs {
 // leaves them bit-identical to sums over the live cells alone.
 
 // U: cells per thread per round of the streaming phases; UA: of the stencil
-// phase. Kernels pick them by their register budget. PF: threads 0..7 of the
+// phase. Kernels pick them by their register budget. PF: threads 0..8 of the
 // block prefetch the block's next round of every streamed array into L2
 // (one bulk prefetch per array), for meshes whose working set exceeds L2.
+// There bytes count, and PF also moves fewer of them: phi += alpha pv of an
+// iteration is left to the next one's stencil phase, which reads that
+// direction anyway (the last one follows the loop), and the residual of the
+// slice's first a.keep_r cells stays in shared memory (`keep`), since only the
+// update phase uses it. 120x240x168: 128 -> 110 bytes a cell and iteration,
+// 117.9 -> 111.4 us. (L2-resident meshes lose by both: 60x120x84 11.6 -> 12.0.)
 // KEEP: the thread's own cells' x, r, aP and this iteration's q = A p stay
 // in the block's shared memory (`keep`, kKeepArrays x slice-length doubles)
 // for the whole solve: the stencil takes the cell's own aP from there, the
@@ -119,6 +126,7 @@ struct CgArgs {
 // up to 32 * kPerLane blocks; larger grids use the counter form.
 template <bool SYM, int U, int UA, bool PF, class G, bool KEEP = false, bool PQS = false>
 __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
+  static_assert(!(PF && KEEP), "one use of the shared memory");
   const MeshDims& d = a.d;
   const SysF64& s = a.s;
   const Slice own = own_slice(d.n, g.nb, g.bid);
@@ -156,6 +164,8 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
         const bool live = c0 + u * B < own.end;
         const double zv = rv[u] / guard_small(fabs(dv[u]));
         if (live) p0[c0 + u * B] = zv;
+        if (PF && live && c0 + u * B - own.begin < a.keep_r)
+          keep[c0 + u * B - own.begin] = rv[u];
         if (KEEP && live) {
           const int o = c0 + u * B - own.begin;
           kx[o] = x[c0 + u * B];
@@ -175,7 +185,8 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
   bool nan_fill = false;
   if (ok && !(bnorm < kSmall)) {
     double rz = v3[2];
-    double beta = 0.0;
+    double beta = 0.0, alpha = 0.0;
+    bool owed = false;  // PF: phi += alpha pv of the last iteration is still to come
     residual = sqrt(v3[1]) / bnorm;
     if (residual != residual && a.max_iter >= 1) nan_fill = true;
     for (int iter = 1; iter <= a.max_iter && !nan_fill; ++iter) {
@@ -218,20 +229,27 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
           }
         }
       } else {
-        const double bt = beta;
+        const double bt = beta, al = alpha;
+        owed = false;
         auto pnew = [z, pold, bt](int cc) { return z[cc] + bt * pold[cc]; };
         for (int c0 = own.begin + (int)threadIdx.x; c0 < own.end; c0 += B * UA) {
-          if (PF && threadIdx.x < 8) {
+          if (PF && threadIdx.x < 9) {
             const int nl = c0 - (int)threadIdx.x + B * UA, nh = min(nl + B * UA, own.end);
-            const double* arr[8] = {z, pold, aP, A.aE, A.aN, A.aT, z, pold};
-            const int off = threadIdx.x >= 6 ? d.plane : 0;
+            const double* arr[9] = {z, pold, aP, A.aE, A.aN, A.aT, x, z, pold};
+            const int off = threadIdx.x >= 7 ? d.plane : 0;
             l2_prefetch_cells(arr[threadIdx.x], nl + off, nh + off, d.n);
           }
-          double qv[UA], pc[UA];
+          double qv[UA], pc[UA], xn[UA];
 #pragma unroll
           for (int u = 0; u < UA; ++u) {
             const int c = min(c0 + u * B, last);
-            pc[u] = pnew(c);
+            if (PF) {
+              const double po = pold[c];
+              pc[u] = z[c] + bt * po;
+              xn[u] = x[c] + al * po;
+            } else {
+              pc[u] = pnew(c);
+            }
             qv[u] = KEEP ? apply_row_diag<SYM, double>(d, A, kd[c - own.begin], pc[u], pnew, c)
                          : apply_row_with<SYM, double>(d, A, pc[u], pnew, c);
           }
@@ -245,6 +263,7 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
               } else {
                 q[c0 + u * B] = qv[u];
               }
+              if (PF) x[c0 + u * B] = xn[u];
             }
             v1[0] = v1[0] + (live ? pc[u] * qv[u] : 0.0);
           }
@@ -260,16 +279,21 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
       if (!ok) break;
       const double pq = v1[0];
       if (fabs(pq) < kSmall) break;
-      const double alpha = rz / pq;
+      alpha = rz / pq;
+      owed = PF;
       // Phase B: phi += alpha pv; r -= alpha q; r.r; z and r.z (:538-553)
       double v2[2] = {0.0, 0.0};
       for (int c0 = own.begin + (int)threadIdx.x; c0 < own.end; c0 += B * U) {
-        if (PF && threadIdx.x < 5) {
+        if (PF && threadIdx.x < 3) {
           const int nl = c0 - (int)threadIdx.x + B * U, nh = min(nl + B * U, own.end);
-          const double* arr[5] = {pcur, q, aP, x, r};
-          l2_prefetch_cells(arr[threadIdx.x], nl, nh, d.n);
+          const double* arr[3] = {q, aP, r};
+          if (threadIdx.x < 2 || nl - own.begin >= a.keep_r)
+            l2_prefetch_cells(arr[threadIdx.x], nl, nh, d.n);
         }
         double pv[U], qv[U], dv[U], xv[U], rv[U];
+        // (a.keep_r is a whole number of rounds)
+        double* __restrict__ rr =
+            PF && c0 - (int)threadIdx.x - own.begin < a.keep_r ? keep - own.begin : r;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int c = min(c0 + u * B, last);
@@ -281,11 +305,11 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
             xv[u] = kx[o];
             rv[u] = kr[o];
           } else {
-            pv[u] = pcur[c];
+            pv[u] = PF ? 0.0 : pcur[c];
             qv[u] = q[c];
             dv[u] = aP[c];
-            xv[u] = x[c];
-            rv[u] = r[c];
+            xv[u] = PF ? 0.0 : x[c];
+            rv[u] = rr[c];
           }
         }
 #pragma unroll
@@ -300,8 +324,8 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
               kx[c - own.begin] = xn;
               kr[c - own.begin] = rn;
             } else {
-              x[c] = xn;
-              r[c] = rn;
+              if (!PF) x[c] = xn;
+              rr[c] = rn;
             }
             z[c] = zv;
           }
@@ -319,6 +343,10 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
       if (residual != residual && iter < a.max_iter) { nan_fill = true; break; }
       beta = v2[1] / guard_small(rz);
       rz = v2[1];
+    }
+    if (PF && owed && !nan_fill) {  // the last iteration's phi += alpha pv
+      const double* __restrict__ p = (n_iter & 1) ? s.p : s.p2;
+      for (int c = own.begin + (int)threadIdx.x; c < own.end; c += B) x[c] = x[c] + alpha * p[c];
     }
     if (KEEP && !nan_fill) {  // the kept x back to global memory
       for (int c = own.begin + (int)threadIdx.x; c < own.end; c += B) x[c] = kx[c - own.begin];
@@ -349,6 +377,7 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
 // one launch shape.
 template <int MAXB, int U, int UA, bool PF>
 __global__ void __launch_bounds__(MAXB, 1) cg_f64_kernel(CgArgs a) {
+  extern __shared__ __align__(16) double keep_smem[];
   Group g;
   g.counter = a.ws.counter;
   g.err = a.ws.err;
@@ -362,9 +391,9 @@ __global__ void __launch_bounds__(MAXB, 1) cg_f64_kernel(CgArgs a) {
   // (PF) it measured slower (121.4 against 117.9 us per iteration at
   // 120x240x168).
   if (*a.s.asym == 0)
-    cg_body<true, U, UA, PF, Group, false, !PF>(a, g);
+    cg_body<true, U, UA, PF, Group, false, !PF>(a, g, keep_smem);
   else
-    cg_body<false, U, UA, PF, Group, false, !PF>(a, g);
+    cg_body<false, U, UA, PF, Group, false, !PF>(a, g, keep_smem);
 }
 
 // The same solver with the own cells' update operands kept in shared memory
@@ -1184,6 +1213,16 @@ static cudaError_t fill_pq_slots(const GroupWs& ws, int grid, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Shared memory for the kept residual of a prefetching block: more of it starves
+// L1, which the stencil phase reads its neighbours from (120x240x168, us per
+// iteration: none 115.6, 96 KB 111.9, 128 KB 111.4, 160 KB 111.9, 208 KB 176).
+constexpr int kKeptResidual = 128 * 1024;
+constexpr int kPrefetchU = 2;  // cells per thread and round of that variant's update phase
+
+static bool cg_f64_prefetches(int block, long long n) {
+  return block > 512 && l2_prefetch_pays(n);
+}
+
 cudaError_t launch_cg_f64(const MeshDims& d, const SysF64& s, const GroupWs& ws,
                           int max_iter, double tol, uint64_t timeout_ns, int grid,
                           int block, cudaStream_t st) {
@@ -1198,9 +1237,20 @@ cudaError_t launch_cg_f64(const MeshDims& d, const SysF64& s, const GroupWs& ws,
   if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
   if (e == cudaSuccess) e = fill_pq_slots(ws, grid, st);
   if (e != cudaSuccess) return e;
+  const void* k = cg_f64_kernel_ptr(block, d.n);
   void* args[] = {&a};
-  return cudaLaunchCooperativeKernel(cg_f64_kernel_ptr(block, d.n), dim3(grid),
-                                     dim3(block), args, 0, st);
+  if (!cg_f64_prefetches(block, d.n))
+    return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(block), args, 0, st);
+  const int round = kPrefetchU * block;
+  const int chunk = (d.n + grid - 1) / grid;
+  const int want = (chunk + round - 1) / round * round;
+  const int room = kKeptResidual / (int)sizeof(double) / round * round;
+  a.keep_r = want < room ? want : room;
+  const size_t smem = (size_t)a.keep_r * sizeof(double);
+  std::lock_guard<std::mutex> attr_lock(launch_attr_mutex());
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(block), args, smem, st);
 }
 
 cudaError_t launch_cg1_f64(const MeshDims& d, const SysF64& s, const GroupWs& ws,
@@ -1440,7 +1490,7 @@ bool l2_prefetch_pays(long long n) { return (double)n * 128.0 > 96.0e6; }
 const void* cg_f64_kernel_ptr(int block, long long n) {
   if (block <= 256) return (const void*)cg_f64_kernel<256, 4, 4, false>;
   if (block <= 512) return (const void*)cg_f64_kernel<512, 4, 2, false>;
-  if (l2_prefetch_pays(n)) return (const void*)cg_f64_kernel<1024, 2, 1, true>;
+  if (cg_f64_prefetches(block, n)) return (const void*)cg_f64_kernel<1024, kPrefetchU, 1, true>;
   return (const void*)cg_f64_kernel<1024, 2, 1, false>;
 }
 

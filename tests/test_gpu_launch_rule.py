@@ -13,10 +13,15 @@ pytestmark = pytest.mark.gpu
 
 
 # 1 cell beyond 16 x 1,760 (a cluster's capacity is about 28,000), a prime-ish
-# mesh, the last and first meshes around the 200 KB a block
-@pytest.mark.parametrize("dims,kernel", [((30, 44, 24), "KEEP"), ((41, 83, 57), "KEEP"),
-                                         ((69, 139, 98), "KEEP"), ((70, 140, 98), "LOADS")])
-def test_untuned_mesh_launch_matches_oracle(dims, kernel):
+# mesh, the last and first meshes around the 200 KB a block, and meshes of the
+# prefetching kernel (part of the residual kept; a kept residual longer than
+# the last block's slice comes with 1024-thread blocks on a smaller mesh)
+@pytest.mark.parametrize("dims,kernel,block", [((30, 44, 24), "KEEP", 512),
+                                               ((41, 83, 57), "KEEP", 512),
+                                               ((69, 139, 98), "KEEP", 512),
+                                               ((70, 140, 98), "LOADS", 512),
+                                               ((80, 161, 111), "LOADS", 1024)])
+def test_untuned_mesh_launch_matches_oracle(dims, kernel, block):
     import oracle
     eaf, g = pkg(), gen()
     s = g.make_system(*dims, 8, seed=3)
@@ -25,8 +30,26 @@ def test_untuned_mesh_launch_matches_oracle(dims, kernel):
         res, nit, st = cg.solve(s.arrays(), a, 12, 0.0)
         plan, ran = cg.last_launch(), cg.last_kernel()
         assert ran == getattr(cg, "KERNEL_" + kernel)
-    assert plan == (148, 512) and st == 0
+    assert plan == (148, block) and st == 0
     assert (res, nit) == oracle.cg(s, b, 12, 0.0, plan=plan)
+    assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("iters", [0, 1, 2, 7])
+def test_prefetching_kernel_ends_with_its_last_update(iters):
+    """The prefetching kernel applies an iteration's update of x in the next
+    one: solves that end after any number of iterations, warm-started."""
+    import oracle
+    eaf, g = pkg(), gen()
+    dims = (93, 91, 90)  # 761,670 cells: 1024-thread blocks prefetch
+    s = g.make_system(*dims, 8, seed=2)
+    a = np.random.default_rng(1).normal(size=g.halo_shape(*dims))
+    b = a.copy()
+    with eaf.CGSolver(*dims) as cg:
+        cg.set_launch(1024, 148)
+        res, nit, _ = cg.solve(s.arrays(), a, iters, 0.0)
+        plan = cg.last_launch()
+    assert (res, nit) == oracle.cg(s, b, iters, 0.0, plan=plan)
     assert np.array_equal(a, b)
 
 
