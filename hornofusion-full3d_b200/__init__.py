@@ -276,8 +276,9 @@ class CGSolver:
 
     def set_resident(self, mode: int = 1) -> None:
         """One-cluster launches of a mesh that fits keep the system in the
-        cluster's shared memory, the blocks signalling their partials by a
-        cluster barrier (RESIDENT_CLUSTER_BARRIER, default) or mbarrier
+        cluster's shared memory, the blocks pushing z and their partials
+        where a thread's one or two cells fit its registers, else signalling
+        by a cluster barrier (RESIDENT_CLUSTER_BARRIER, default) or mbarrier
         arrivals (RESIDENT_MBARRIER), or run the global-memory cluster kernel
         (RESIDENT_OFF); all give the same bits."""
         check(self._lib.eaf_cg_set_resident(self._h, int(mode)), "set_resident")

@@ -147,9 +147,10 @@ SolverLaunch choose_launch(int nr, int nth, int nz, int sms, int req_block, int 
   bool spread = false;
   if (automatic && f64 && form == EAF_CG_FORM_REFERENCE && !tuned && req_cluster == 0) {
     // A small mesh outside the table: one cluster that keeps the system in
-    // its shared memory (8 blocks up to 8192 cells, else 16), one cell per
-    // thread up to 640 cells a block, else two.
-    const int cs = n <= 8192 ? 8 : 16;
+    // its shared memory, one cell per thread up to 640 cells a block, else two;
+    // 8 blocks while they hold it at one cell a thread, else 16 (14x28x20,
+    // 7,840 cells, us per iteration: 2.6 on 8, 2.2 on 16).
+    const int cs = n <= 8 * 640 ? 8 : 16;
     const long long per = (n + cs - 1) / cs;
     long long t = per <= 640 ? per : (per + 1) / 2;
     t = ((t + 31) / 32) * 32;
@@ -232,7 +233,7 @@ cudaError_t launch_f64_solver(const SolverLaunch& L, int resident, const MeshDim
                               int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st) {
   if (runs_resident(L, d.n, resident != 0))
     return launch_cg_f64_dsm(d, s, ws, max_iter, tol, L.block, L.cluster, st,
-                             resident == 2 ? kDsmSignalMbarrier : kDsmSignalClusterBarrier,
+                             resident == 2 ? kDsmSignalMbarrier : kDsmSignalDefault,
                              timeout_ns);
   if (L.cluster > 1 || L.slots)
     return launch_cg_f64_cluster(d, s, ws, ws.part, slot_doubles, max_iter, tol, timeout_ns,

@@ -20,10 +20,11 @@
 //     cluster all-reduce with one cluster (the oracle's plan (C, B, C)), so
 //     the solve is bit-identical to cg_cluster_kernel on the same launch
 //     shape and to the oracle. The signal is either a full cluster barrier
-//     (the default: measured faster, 3.4 against 3.9 us per iteration at
-//     12x24x16) or a remote arrival on an mbarrier of each block (release at
-//     cluster scope, one arrival per block and phase, barriers
-//     double-buffered by all-reduce parity).
+//     (3.4 us per iteration at 12x24x16) or a remote arrival on an mbarrier of
+//     each block (release at cluster scope, one arrival per block and phase,
+//     barriers double-buffered by all-reduce parity; 3.9 us).
+// Where a thread's cells fit its registers, the default is the pushed form
+// (cg_push_kernel, below): 1.8 us.
 //
 // Global memory is read once (the packed system) and written once (x and
 // the result). There is no global synchronisation and no wait that another
@@ -31,9 +32,11 @@
 // and reaches every cluster barrier on every path (the exit decisions depend
 // only on the totals, which all blocks fold identically).
 #include <math.h>
+#include <stddef.h>
 
 #include "cg_kernels.h"
 #include "cluster_red.cuh"
+#include "recipdiv.cuh"
 #include "stencil.cuh"
 
 namespace eaf {
@@ -57,6 +60,7 @@ struct DsmArgs {
   double tol;
   uint64_t timeout_ns;
   int chunk;     // cells per block
+  int reach;     // blocks on either side that hold neighbours (pushed form)
   FastDiv fd_chunk;
 };
 
@@ -398,6 +402,556 @@ __global__ void __launch_bounds__(1024, 1) cg_dsm_kernel(DsmArgs a) {
   cluster_sync_all();
 }
 
+// ---------------------------------------------------------------------------
+// Pushed form: a thread holds its one or two cells in registers for the whole
+// solve -- coefficients, x, r, z, q, its direction and, instead of re-reading
+// z and the old direction of the six neighbours, their directions, which it
+// advances itself (p_nb = z_nb + beta p_nb, the owner's own operation). What an
+// iteration exchanges is the new z and the blocks' partials, and both are
+// PUSHED, completing bytes on an mbarrier of the receiving block: the partials
+// by st.async, a block's slice of z by one bulk copy to each block within a
+// z-plane of it (every neighbour of a cell is less than a plane away). A block
+// keeps the slices it receives beside its own, so all its reads are local.
+// Measured on 16 blocks of 288 threads, cycles: remote stores and a releasing
+// cluster barrier 1035, pushed exchange 370; six remote loads a thread 930.
+// (z by one st.async per cell and remote neighbour was no faster than the
+// bulk copies and needs the addresses in registers.) us per iteration, cluster
+// barrier -> pushed: 10x20x12 2.9 -> 1.6, 12x24x16 3.4 -> 1.8, 18x36x24
+// 4.5 -> 2.8. What is left is latency: two reductions of two butterflies each,
+// two exchanges and one division chain an iteration.
+//
+// Order. Two exchanges an iteration, each on its own barrier: p.q after the
+// stencil phase, (r.r, r.z) and z after the update phase. A block's partial
+// and its copies follow a block barrier behind everything its threads read
+// and wrote, so: received slices and partial slots are overwritten, and the
+// own z behind an earlier copy rewritten, only after every block has this
+// block's next partial; a barrier's next phase cannot receive bytes before
+// this one was waited for by every thread here (a block two exchanges ahead
+// would need this block's partial between). The arithmetic and the
+// association are dsm_body's.
+// ---------------------------------------------------------------------------
+struct PushSmem {
+  // Block partials by rank, as many doubles each as the sums they carry
+  // (preamble: three and a pad).
+  double pq[kMaxClusterSize], rz[kMaxClusterSize][2], pre[kMaxClusterSize][4];
+  double warp[kClusterSlotsNV][32];
+  double zero;       // z of a missing neighbour
+  double dummy;      // where cells beyond the slice leave theirs
+  uint64_t bar[2];
+};
+static_assert(offsetof(PushSmem, rz) == 8 * kMaxClusterSize &&
+                  offsetof(PushSmem, pre) == 24 * kMaxClusterSize &&
+                  offsetof(PushSmem, warp) == 56 * kMaxClusterSize,
+              "the offsets that push_allsum uses");
+
+// What a block's all-reduces need, set up once (shared-memory addresses).
+struct Pusher {
+  int rank;
+  uint32_t phases;             // completion parity expected next, bit per barrier
+  uint32_t smem, bar;          // this block's PushSmem and barriers
+  uint32_t to_smem, to_bar;    // those of lane's target block (lane & 15)
+  uint32_t z_bytes;            // bytes of z a block receives per exchange
+  uint32_t z_src, z_dst, z_len, z_bar;  // last warp: lane's copy of z
+  int* err;
+  uint64_t timeout_ns;
+};
+
+__device__ __forceinline__ void st_async_f64(uint32_t dst, double v, uint32_t bar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+      "l"(__double_as_longlong(v)), "r"(bar)
+      : "memory");
+}
+// (the writers of the source have passed a proxy fence and a block barrier)
+__device__ __forceinline__ void push_bulk(uint32_t dst, uint32_t src, uint32_t bytes,
+                                          uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+      "[%3];" ::"r"(dst),
+      "r"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+
+// The slices of z in a block's shared memory: slot s holds that of block
+// rank - reach + s; a slot is `pad` doubles (the slice, to 16 bytes).
+struct Slices {
+  int reach, pad;
+  uint32_t base;
+  __device__ __forceinline__ uint32_t slot(int rank, int owner) const {
+    return base + 8u * (uint32_t)((owner - rank + reach) * pad);
+  }
+  __device__ __forceinline__ uint32_t bytes(const DsmArgs& a, int owner) const {
+    const int cells = max(0, min(a.chunk, a.d.n - owner * a.chunk));
+    return 8u * (uint32_t)((cells + 1) & ~1);
+  }
+};
+__device__ __forceinline__ double ld_shared_f64(uint32_t a) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// Sums of the warp's NV values, by the xor butterfly (steps 16, 8, 4, 2, 1);
+// HALF: only lanes 0..15 hold values, the others zeros, and step 16, which
+// would add them, is left out (x + 0 is x for every sum but -0, and no sum
+// here is -0 where it matters). Two values share the steps after the first:
+// each half of the warp goes on with one of them. Value m is valid in lane
+// 16 m (one value: every lane).
+template <int NV, bool HALF>
+__device__ __forceinline__ double warp_sums(const double (&v)[NV], int lane) {
+  static_assert(NV <= 2, "one value per half");
+  const unsigned all = 0xffffffffu;
+  double t;
+  if (NV == 1) {
+    t = v[0];
+    if (!HALF) t = t + __shfl_xor_sync(all, t, 16);
+  } else {
+    const bool up = lane >= 16;
+    const double got = __shfl_xor_sync(all, up ? v[0] : v[NV - 1], 16);
+    const double mine = up ? v[NV - 1] : v[0];
+    t = HALF ? (up ? got : mine) : mine + got;
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) t = t + __shfl_xor_sync(all, t, o);
+  return t;
+}
+
+// Opens the next phase of a barrier: it completes with `bytes` pushed.
+__device__ __forceinline__ void push_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void ld_shared_pair(uint32_t a, double& v, double& w) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v), "=d"(w) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void st_shared_f64(uint32_t a, double v) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// Offsets in a PushSmem, and the doubles a block's sums take there.
+constexpr uint32_t kAtPq = 0, kAtRz = 8 * kMaxClusterSize, kAtPre = 24 * kMaxClusterSize,
+                   kAtWarp = 56 * kMaxClusterSize;
+
+// All-reduce of NV sums over the cluster: warp sums, block sums (warp 0)
+// pushed to every block, with KIND 1 also z (the last warp); then every thread
+// waits for the partials of the (at most) CMAX blocks, whose slots beyond the
+// cluster's size hold zeros, and folds them in rank order. Two values are
+// pushed by the two halves of warp 0. The barrier's next phase, which will
+// carry `next` bytes, is opened on the way out. False if the wait gave up; a
+// block leaves as one.
+template <int NV, int KIND, int CMAX>
+__device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t next, Pusher& x) {
+  constexpr int kPairs = (NV + 1) / 2;  // values go two by two
+  constexpr int kTwo = NV >= 2 ? 2 : 1;
+  constexpr uint32_t kStride = 8 * (NV <= 2 ? NV : 4);
+  constexpr uint32_t kAt = NV == 1 ? kAtPq : NV == 2 ? kAtRz : kAtPre;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int h = 0; h < kPairs; ++h) {
+    double in[kTwo];
+#pragma unroll
+    for (int m = 0; m < kTwo; ++m) in[m] = 2 * h + m < NV ? v[2 * h + m < NV ? 2 * h + m : 0] : 0.0;
+    const double t = warp_sums<kTwo, false>(in, lane);
+    if ((lane & 15) == 0)
+      st_shared_f64(x.smem + kAtWarp + 8u * (uint32_t)(32 * (2 * h + (kTwo - 1) * (lane >> 4)) + w), t);
+  }
+  if (KIND == 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  if (KIND == 1 && w == nw - 1) {
+    if (x.z_len) push_bulk(x.z_dst, x.z_src, x.z_len, x.z_bar);
+    __syncwarp();
+  }
+  if (w == 0) {
+    const uint32_t dst = x.to_smem + kAt + kStride * (uint32_t)x.rank + 8u * (kTwo - 1) * (lane >> 4);
+    const bool pushes = (lane & 15) < C && (kTwo == 2 || lane < 16);
+#pragma unroll
+    for (int h = 0; h < kPairs; ++h) {
+      double in[kTwo];
+#pragma unroll
+      for (int m = 0; m < kTwo; ++m)
+        in[m] = lane < nw && 2 * h + m < NV
+                    ? ld_shared_f64(x.smem + kAtWarp + 8u * (uint32_t)(32 * (2 * h + m) + lane))
+                    : 0.0;
+      const double t = nw <= 16 ? warp_sums<kTwo, true>(in, lane) : warp_sums<kTwo, false>(in, lane);
+      if (pushes && (2 * h + 1 < NV || lane < 16))
+        st_async_f64(dst + 16u * h, t, x.to_bar + 8u * KIND);
+    }
+    __syncwarp();
+  }
+  const uint32_t bar = x.bar + 8u * KIND;
+  const uint32_t want = (x.phases >> KIND) & 1u;
+  x.phases ^= 1u << KIND;
+  bool ok = true;
+  if (!mbar_test_cluster(bar, want)) {
+    const uint64_t t0 = global_ns();
+    uint32_t spins = 0;
+    while (!mbar_test_cluster(bar, want)) {
+      if ((++spins & 255u) == 0) {
+        if (ld_volatile_i32(x.err) != 0) { ok = false; break; }
+        if (global_ns() - t0 > x.timeout_ns) {
+          atomicCAS(x.err, 0, (int)EAF_ETIMEOUT);
+          ok = false;
+          break;
+        }
+      }
+    }
+  }
+  ok = __syncthreads_and(ok) != 0;
+  if (threadIdx.x == blockDim.x - 1) push_expect(bar, next);
+  const uint32_t part = x.smem + kAt;
+  if (NV == 1) {
+    double t[CMAX];
+#pragma unroll
+    for (int r = 0; r < CMAX; r += 2) ld_shared_pair(part + 8u * r, t[r], t[r + 1]);
+    v[0] = t[0];
+#pragma unroll
+    for (int r = 1; r < CMAX; ++r) v[0] = v[0] + t[r];
+  } else if (NV == 2) {
+    ld_shared_pair(part, v[0], v[NV - 1]);
+#pragma unroll
+    for (int r0 = 1; r0 < CMAX; r0 += 8) {
+      double t[8], u[8];
+#pragma unroll
+      for (int r = r0; r < r0 + 8 && r < CMAX; ++r)
+        ld_shared_pair(part + 16u * r, t[r - r0], u[r - r0]);
+#pragma unroll
+      for (int r = r0; r < r0 + 8 && r < CMAX; ++r) {
+        v[0] = v[0] + t[r - r0];
+        v[NV - 1] = v[NV - 1] + u[r - r0];
+      }
+    }
+  } else {
+    for (int m = 0; m < NV; ++m) {
+      double t = ld_shared_f64(part + 8u * m);
+#pragma unroll 1
+      for (int r = 1; r < CMAX; ++r) t = t + ld_shared_f64(part + kStride * r + 8u * m);
+      v[m] = t;
+    }
+  }
+  return ok;
+}
+
+// Neighbour in direction d (kW..kT) of compact cell (i, j, k), or -1 at an r
+// or z wall; its direction back is d ^ 1.
+__device__ __forceinline__ int neighbour(const MeshDims& d, int c, int i, int j, int k, int dir) {
+  switch (dir) {
+    case kW: return i > 0 ? c - 1 : -1;
+    case kE: return i < d.nr - 1 ? c + 1 : -1;
+    case kS: return j > 0 ? c - d.nr : c + (d.nth - 1) * d.nr;
+    case kN: return j < d.nth - 1 ? c + d.nr : c - (d.nth - 1) * d.nr;
+    case kB: return k > 0 ? c - d.plane : -1;
+    default: return k < d.nz - 1 ? c + d.plane : -1;
+  }
+}
+
+// What only the update phase uses of a thread's cells: x, the Jacobi divisor
+// and its reciprocal; in registers for one cell, in shared memory for two,
+// whose 128 registers would spill.
+template <int R>
+struct Own {
+  double v[3];
+  __device__ __forceinline__ void init(uint32_t) {}
+  __device__ __forceinline__ void set(int, double x, double d, double y) {
+    v[0] = x; v[1] = d; v[2] = y;
+  }
+  __device__ __forceinline__ double x(int) const { return v[0]; }
+  __device__ __forceinline__ double dv(int) const { return v[1]; }
+  __device__ __forceinline__ double dy(int) const { return v[2]; }
+  __device__ __forceinline__ void set_x(int, double x) { v[0] = x; }
+};
+template <>
+struct Own<2> {
+  uint32_t at, row;  // three rows of 2 B doubles
+  __device__ __forceinline__ void init(uint32_t base) {
+    at = base + 8u * threadIdx.x;
+    row = 16u * blockDim.x;
+  }
+  __device__ __forceinline__ uint32_t cell(int m) const { return at + (m ? row / 2 : 0u); }
+  __device__ __forceinline__ void set(int m, double x, double d, double y) {
+    st_shared_f64(cell(m), x);
+    st_shared_f64(cell(m) + row, d);
+    st_shared_f64(cell(m) + 2 * row, y);
+  }
+  __device__ __forceinline__ double x(int m) const { return ld_shared_f64(cell(m)); }
+  __device__ __forceinline__ double dv(int m) const { return ld_shared_f64(cell(m) + row); }
+  __device__ __forceinline__ double dy(int m) const { return ld_shared_f64(cell(m) + 2 * row); }
+  __device__ __forceinline__ void set_x(int m, double x) { st_shared_f64(cell(m), x); }
+};
+
+template <bool SYM, int R, int CMAX>
+__device__ void push_body(const DsmArgs& a, double* sm, PushSmem& ps, int C, int rank) {
+  const uint32_t own_smem =
+      smem_addr(sm + (size_t)(2 * a.reach + 1) * ((a.chunk + 1) & ~1));
+  const MeshDims& d = a.d;
+  const SysF64& s = a.s;
+  const int begin = min(d.n, rank * a.chunk), end = min(d.n, begin + a.chunk);
+  const int B = blockDim.x;
+  int* err = a.ws.err;
+  Slices zs;
+  zs.reach = a.reach;
+  zs.pad = (a.chunk + 1) & ~1;
+  zs.base = smem_addr(sm);
+  const uint32_t own_z = zs.slot(rank, rank);
+  Pusher px;
+  {
+    const int lane = threadIdx.x & 31, to = rank - zs.reach + lane;
+    px.rank = rank;
+    px.phases = 0;
+    px.smem = smem_addr(&ps);
+    px.bar = smem_addr(&ps.bar[0]);
+    px.to_smem = cluster_map(px.smem, (uint32_t)min(lane & 15, C - 1));
+    px.to_bar = cluster_map(px.bar, (uint32_t)min(lane & 15, C - 1));
+    px.z_bytes = 0;
+    for (int b = max(0, rank - zs.reach); b <= min(C - 1, rank + zs.reach); ++b)
+      if (b != rank) px.z_bytes += zs.bytes(a, b);
+    const bool sends = lane <= 2 * zs.reach && to >= 0 && to < C && to != rank;
+    px.z_len = sends ? zs.bytes(a, rank) : 0u;
+    px.z_src = own_z;
+    px.z_dst = sends ? cluster_map(zs.slot(to, rank), (uint32_t)to) : 0u;
+    px.z_bar = sends ? cluster_map(px.bar + 8u, (uint32_t)to) : 0u;
+    px.err = err;
+    px.timeout_ns = a.timeout_ns;
+  }
+  const uint32_t zero = smem_addr(&ps.zero);
+  const uint32_t pq_bytes = 8u * (uint32_t)C, rz_bytes = 16u * (uint32_t)C + px.z_bytes;
+  if (threadIdx.x == 0) {
+    push_expect(px.bar, pq_bytes);
+    push_expect(px.bar + 8u, 24u * (uint32_t)C + px.z_bytes);
+  }
+  // Every cell of this thread; a dead one (beyond the slice) sums zeros.
+  double ap[R], al[R][6], r[R], z[R], p[R], q[R], pn[R][6];
+  Own<R> own;
+  own.init(own_smem);
+  uint32_t from[R][6], z_at[R];
+  bool live[R], d_ok[R];
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    const int c = begin + (int)threadIdx.x + m * B;
+    live[m] = c < end;
+    ap[m] = r[m] = z[m] = p[m] = q[m] = 0.0;
+    double xv = 0.0, dv = 1.0, dy = 1.0;
+    d_ok[m] = true;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      al[m][e] = pn[m][e] = 0.0;
+      from[m][e] = zero;
+    }
+    z_at[m] = smem_addr(&ps.dummy);
+    if (live[m]) {
+      z_at[m] = own_z + 8u * (uint32_t)(c - begin);
+      int i, j, k;
+      cell_ijk(d, c, i, j, k);
+      ap[m] = s.aP[c];
+      xv = s.x[c];
+      r[m] = s.r[c];
+      dv = guard_small(fabs(ap[m]));
+      d_ok[m] = exp_in_safe_range(dv);
+      dy = d_ok[m] ? 1.0 / dv : 0.0;
+#pragma unroll
+      for (int e = 0; e < 6; ++e) {
+        const int nb = neighbour(d, c, i, j, k, e);
+        const double* lower = e == kW ? s.aE : e == kS ? s.aN : s.aT;  // symmetric form
+        const double* own = e == kW   ? s.aW
+                            : e == kE ? s.aE
+                            : e == kS ? s.aS
+                            : e == kN ? s.aN
+                            : e == kB ? s.aB
+                                      : s.aT;
+        if (SYM)
+          al[m][e] = nb < 0 ? 0.0 : (e & 1) ? own[c] : lower[nb];
+        else
+          al[m][e] = own[c];
+        if (nb < 0) continue;
+        const int owner = (int)a.fd_chunk.div((uint32_t)nb);
+        from[m][e] = zs.slot(rank, owner) + 8u * (uint32_t)(nb - owner * a.chunk);
+      }
+    }
+    own.set(m, xv, dv, dy);
+  }
+  // z = r / max(|aP|, SMALL) of the thread's cells, kept and stored; the
+  // quotient by the stored reciprocal (recipdiv.cuh), `/` outside its range.
+  auto precondition = [&](int m) {
+    const double dv = own.dv(m), dy = own.dy(m);
+    const double t = r[m], q0 = t * dy;
+    double zv = __fma_rn(__fma_rn(-q0, dv, t), dy, q0);
+    if (!(d_ok[m] & (exp_in_safe_range(t) | (__double_as_longlong(t) == 0)))) {
+      asm volatile("" ::: "memory");  // (keeps the division in its own branch)
+      zv = t / dv;
+    }
+    z[m] = zv;
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(z_at[m]), "d"(zv) : "memory");
+  };
+
+  // Preamble (src/mod_solver_3d.f90:515-530).
+  double v3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    precondition(m);
+    const double bv = live[m] ? s.b[begin + threadIdx.x + m * B] : 0.0;
+    v3[0] = v3[0] + bv * bv;
+    v3[1] = v3[1] + r[m] * r[m];
+    v3[2] = v3[2] + r[m] * z[m];
+  }
+  bool ok = push_allsum<3, 1, CMAX>(v3, C, rz_bytes, px);
+  const double bnorm = sqrt(v3[0]);
+  double residual = 0.0, rr = 0.0;
+  int n_iter = 0;
+  bool nan_fill = false;
+  if (ok && !(bnorm < kSmall)) {
+    double rz = v3[2], beta = 0.0;
+    rr = v3[1];
+    residual = sqrt(rr) / bnorm;
+    // A r.r above this cannot give a residual below tol (the square root and
+    // the quotient of the exit test, some 250 cycles, are then left out); out
+    // of range, the test is always made.
+    const double lim = (a.tol * bnorm) * (a.tol * bnorm) * (1.0 + 1e-12);
+    const double surely_above = lim > 1e-290 && lim < 1e290 ? lim : lim == 0.0 && a.tol == 0.0
+                                                                        ? 0.0
+                                                                        : HUGE_VAL;
+    if (residual != residual && a.max_iter >= 1) nan_fill = true;
+    for (int iter = 1; iter <= a.max_iter && !nan_fill; ++iter) {
+      // p = z + beta p (own and neighbours), q = A p, p.q. A missing
+      // neighbour's direction stays zero: the symmetric form's link to it is
+      // zero too (the term the reference's loop does not have changes
+      // nothing), the general form's multiplies a zero. Only a beta that is
+      // not finite would turn it into NaN.
+      double v1[1] = {0.0};
+      const bool first = iter == 1, finite = isfinite(beta);
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        double zn[6];
+#pragma unroll
+        for (int e = 0; e < 6; ++e) zn[e] = ld_shared_f64(from[m][e]);
+        if (first) {
+          p[m] = z[m];
+#pragma unroll
+          for (int e = 0; e < 6; ++e) pn[m][e] = zn[e];
+        } else {
+          p[m] = z[m] + beta * p[m];
+#pragma unroll
+          for (int e = 0; e < 6; ++e) pn[m][e] = zn[e] + beta * pn[m][e];
+          if (!finite) {
+            asm volatile("" ::: "memory");
+#pragma unroll
+            for (int e = 0; e < 6; ++e)
+              if (from[m][e] == zero) pn[m][e] = 0.0;
+            if (!live[m]) p[m] = 0.0;
+          }
+        }
+        double y = ap[m] * p[m];
+#pragma unroll
+        for (int e = 0; e < 6; ++e) y = y - al[m][e] * pn[m][e];
+        q[m] = y;
+        v1[0] = v1[0] + p[m] * y;
+      }
+      if (!(ok = push_allsum<1, 0, CMAX>(v1, C, pq_bytes, px))) break;
+      const double pq = v1[0];
+      if (fabs(pq) < kSmall) break;
+      const double alpha = rz / pq;
+      // beta's reciprocal, beside that division and off its own chain
+      const double rz_g = guard_small(rz);
+      const bool rz_ok = exp_in_safe_range(rz_g);
+      const double rz_y = rz_ok ? 1.0 / rz_g : 0.0;
+      const bool steps = isfinite(alpha);
+      double v2[2] = {0.0, 0.0};
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        own.set_x(m, own.x(m) + alpha * p[m]);
+        r[m] = r[m] - alpha * q[m];
+        if (!steps && !live[m]) r[m] = 0.0;  // (0 * Inf)
+        precondition(m);
+        v2[0] = v2[0] + r[m] * r[m];
+        v2[1] = v2[1] + r[m] * z[m];
+      }
+      if (!(ok = push_allsum<2, 1, CMAX>(v2, C, rz_bytes, px))) break;
+      rr = v2[0];
+      n_iter = iter;
+      if (!(rr > surely_above)) {
+        residual = sqrt(rr) / bnorm;
+        if (residual < a.tol) break;
+        if (residual != residual && iter < a.max_iter) { nan_fill = true; break; }
+      }
+      beta = div_by_recip(v2[1], rz_g, rz_y, rz_ok);
+      rz = v2[1];
+    }
+  }
+  if (n_iter > 0) residual = sqrt(rr) / bnorm;
+  const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll
+  for (int m = 0; m < R; ++m)
+    if (live[m]) s.x[begin + threadIdx.x + m * B] = nan_fill ? qnan : own.x(m);
+  if (nan_fill) {
+    residual = qnan;
+    n_iter = a.max_iter;
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    SolveResult* res = a.ws.result;
+    const int e = ld_volatile_i32(err);
+    res->status = e != 0 ? e : (isfinite(residual) ? EAF_OK : EAF_ENONFINITE);
+    res->n_iter = n_iter;
+    res->n_outer = 0;
+    res->sym = SYM ? 1 : 0;
+    res->residual = residual;
+    res->bnorm = bnorm;
+  }
+}
+
+// Threads of a block whose cells (one or two each) fit its registers: one
+// cell in 96 (640 threads) or more, two in 128.
+constexpr int kPushBlock1 = 640, kPushBlock2 = 512, kPushSmall = 384;
+
+template <int R, int MAXB, int CMAX>
+__global__ void __launch_bounds__(MAXB, 1) cg_push_kernel(DsmArgs a) {
+  extern __shared__ __align__(16) double push_smem[];
+  __shared__ __align__(16) PushSmem ps;
+  const int rank = (int)cluster_ctarank(), C = (int)cluster_nctarank();
+  for (int i = threadIdx.x; i < 7 * kMaxClusterSize; i += blockDim.x)
+    ps.pq[i] = 0.0;  // (and rz, pre behind it)
+  if (threadIdx.x == 0) {
+    ps.zero = 0.0;
+    for (int b = 0; b < 2; ++b)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&ps.bar[b]))
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // Every block's barriers exist before any block pushes.
+  cluster_sync_all();
+  if (*a.s.asym == 0)
+    push_body<true, R, CMAX>(a, push_smem, ps, C, rank);
+  else
+    push_body<false, R, CMAX>(a, push_smem, ps, C, rank);
+  // No block leaves while another may still push into its memory.
+  cluster_sync_all();
+}
+
+// Cells per thread of the pushed form for blocks of `block` threads, 0 where
+// it does not apply: more cells than registers, or slices much thinner than a
+// plane, whose z would go to too many blocks.
+constexpr int kPushReach = 3;
+int push_reach(const MeshDims& d, int chunk) { return (d.plane + chunk - 1) / chunk; }
+int push_cells(const MeshDims& d, int chunk, int block) {
+  const int r = (chunk + block - 1) / block;
+  if (push_reach(d, chunk) > kPushReach) return 0;
+  return r == 1 && block <= kPushBlock1 ? 1 : r == 2 && block <= kPushBlock2 ? 2 : 0;
+}
+template <int CMAX>
+const void* push_kernel_of(int cells, int block) {
+  if (cells == 1)
+    return block <= kPushSmall ? (const void*)cg_push_kernel<1, kPushSmall, CMAX>
+                               : (const void*)cg_push_kernel<1, kPushBlock1, CMAX>;
+  return block <= kPushSmall ? (const void*)cg_push_kernel<2, kPushSmall, CMAX>
+                             : (const void*)cg_push_kernel<2, kPushBlock2, CMAX>;
+}
+const void* push_kernel(int cells, int block, int cluster) {
+  return cluster <= 8 ? push_kernel_of<8>(cells, block)
+                      : push_kernel_of<kMaxClusterSize>(cells, block);
+}
+size_t push_smem_bytes(int reach, int chunk, int cells, int block) {
+  const size_t slices = (size_t)(2 * reach + 1) * ((chunk + 1) & ~1);
+  return (slices + (cells == 2 ? (size_t)6 * block : 0)) * sizeof(double);
+}
+
 size_t dsm_smem_bytes(int chunk) { return (size_t)kDsmArrays * chunk * sizeof(double); }
 
 }  // namespace
@@ -464,9 +1018,13 @@ cudaError_t launch_cg_f64_dsm(const MeshDims& d, const SysF64& s, const GroupWs&
   a.timeout_ns = timeout_ns;
   a.chunk = (d.n + cluster - 1) / cluster;
   a.fd_chunk = FastDiv((uint32_t)a.chunk);
-  const size_t smem = dsm_smem_bytes(a.chunk);
-  const void* k = signal == kDsmSignalMbarrier ? (const void*)cg_dsm_kernel<true>
-                                                : (const void*)cg_dsm_kernel<false>;
+  // The default signalling pushes where a thread's cells fit its registers.
+  const int cells = signal == kDsmSignalMbarrier ? 0 : push_cells(d, a.chunk, block);
+  a.reach = push_reach(d, a.chunk);
+  const size_t smem = cells ? push_smem_bytes(a.reach, a.chunk, cells, block) : dsm_smem_bytes(a.chunk);
+  const void* k = cells ? push_kernel(cells, block, cluster)
+                  : signal == kDsmSignalMbarrier ? (const void*)cg_dsm_kernel<true>
+                                                 : (const void*)cg_dsm_kernel<false>;
   std::lock_guard<std::mutex> attr_lock(launch_attr_mutex());
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
