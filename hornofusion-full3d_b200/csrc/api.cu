@@ -72,9 +72,7 @@ static void free_handle(eaf_cg* h) {
   cudaFree(h->ws.part);
   cudaFree(h->ws.counter);
   cudaFree(h->ws.err);
-  cudaFree(h->ws.result);
   cudaFree(h->tdma_mbox);
-  cudaFree(h->tdma_fac);
   cudaFree(h->pc_d);
   cudaFree(h->pc_i);
   cudaFree(h->asm_d);
@@ -328,8 +326,12 @@ int eaf_cg_create_mesh(eaf_cg_t* out, int nr, int nth, int nz, int is_parallel,
   alloc((void**)&h->ws.part, sizeof(double) * kPartTableDoubles(h));
   alloc((void**)&h->ws.counter, sizeof(unsigned long long));
   alloc((void**)&h->ws.err, sizeof(int));
-  alloc((void**)&h->ws.result, sizeof(SolveResult));
-  if (e == cudaSuccess) e = cudaHostAlloc((void**)&h->res_h, sizeof(SolveResult), 0);
+  // The kernels write a solve's result (and, in the second record, the
+  // assembly's residual) straight to pinned host memory: some fifty bytes,
+  // instead of a copy behind the last kernel.
+  if (e == cudaSuccess)
+    e = cudaHostAlloc((void**)&h->res_h, 2 * sizeof(SolveResult), cudaHostAllocMapped);
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&h->ws.result, h->res_h, 0);
   for (int i = 0; i < 6 && e == cudaSuccess; ++i) e = cudaEventCreate(&h->ev[i]);
   if (e != cudaSuccess) {
     set_error("eaf_cg_create", e);
@@ -559,8 +561,6 @@ int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts&
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(eaf::launch_unpack_f64(h->d, h->s.x, phi, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[4], h->st));
-  EAF_CUDA(cudaMemcpyAsync(h->res_h, h->ws.result, sizeof(SolveResult),
-                           cudaMemcpyDeviceToHost, h->st));
   h->last_kernels = 3;
   return EAF_OK;
 }

@@ -21,13 +21,13 @@ namespace {
 // Line-by-line TDMA sweeps and the transport residual on the handle's mesh.
 // ---------------------------------------------------------------------------
 int enqueue_tdma(eaf_cg* h, const HaloInputs& in, double* phi, int n_sweep) {
-  if (!h->tdma_mbox) {
+  if (!h->tdma_mbox) {  // the mailboxes and the records, in one allocation
+    const size_t mbox =
+        (eaf::tdma_mailbox_doubles(h->nr, h->nth, h->nz) + 31) / 32 * 32;
     EAF_CUDA(cudaMalloc((void**)&h->tdma_mbox,
-                        sizeof(double) * eaf::tdma_mailbox_doubles(h->nr, h->nth, h->nz)));
-  }
-  if (!h->tdma_fac) {
-    EAF_CUDA(cudaMalloc((void**)&h->tdma_fac,
-                        sizeof(double) * eaf::tdma_factor_doubles(h->nr, h->nth, h->nz)));
+                        sizeof(double) *
+                            (mbox + eaf::tdma_factor_doubles(h->nr, h->nth, h->nz))));
+    h->tdma_fac = h->tdma_mbox + mbox;
   }
   eaf::tdma_launch_shape(h->nr, h->nth, h->nz, h->sms, &h->last_grid, &h->last_block);
   h->last_cluster = 1;
@@ -67,8 +67,6 @@ int run_residual(eaf_cg* h, const HaloInputs& in, const double* phi, double* res
   EAF_CUDA(cudaEventRecord(h->ev[2], h->st));
   EAF_CUDA(eaf::launch_residual_f64(in, phi, h->d, h->ws, h->timeout_ns, grid, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
-  EAF_CUDA(cudaMemcpyAsync(h->res_h, h->ws.result, sizeof(SolveResult),
-                           cudaMemcpyDeviceToHost, h->st));
   EAF_CUDA(cudaStreamSynchronize(h->st));
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, h->ev[2], h->ev[3]) == cudaSuccess) h->last_kernel_ms = ms;
@@ -163,11 +161,9 @@ int run_assemble(eaf_cg* h, const eaf_assembly_fields_t& f) {
                         sizeof(double) * eaf::assembly_scratch_doubles(h->nr, h->nth, h->nz)));
   }
   EAF_CUDA(cudaEventRecord(h->ev[2], h->st));
-  EAF_CUDA(eaf::launch_assemble_f64(f, h->nr, h->nth, h->nz, h->asm_s, h->st));
+  EAF_CUDA(eaf::launch_assemble_f64(f, h->nr, h->nth, h->nz, h->asm_s,
+                                    &h->ws.result[1].residual, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
-  EAF_CUDA(cudaMemcpyAsync(&h->res_h->residual,
-                           eaf::assembly_result(h->asm_s, h->nr, h->nth, h->nz),
-                           sizeof(double), cudaMemcpyDeviceToHost, h->st));
   h->last_kernels = 4;
   return EAF_OK;
 }
@@ -283,7 +279,8 @@ int run_step(eaf_cg* h, const eaf_assembly_fields_t& d, double alpha_p, int max_
   for (int i = 0; i < 2; ++i)
     if (!h->step_ev[i]) EAF_CUDA(cudaEventCreate(&h->step_ev[i]));
   EAF_CUDA(cudaEventRecord(h->step_ev[0], h->st));
-  EAF_CUDA(eaf::launch_assemble_f64(d, h->nr, h->nth, h->nz, h->asm_s, h->st));
+  EAF_CUDA(eaf::launch_assemble_f64(d, h->nr, h->nth, h->nz, h->asm_s,
+                                    &h->ws.result[1].residual, h->st));
   HaloInputs in = {d.aW, d.aE, d.aS, d.aN, d.aB, d.aT, d.aP, d.Su, d.pp};
   SolveOpts o = {false, max_iter, 0, tol, 0.0};
   int rc = enqueue_solve(h, in, d.pp, o);
@@ -313,9 +310,7 @@ int run_step(eaf_cg* h, const eaf_assembly_fields_t& d, double alpha_p, int max_
   EAF_CUDA(cudaEventRecord(h->step_ev[1], h->st));
   const int st = finish_solve(h, false, cg_res, n_iter, nullptr);  // synchronises
   if (st != EAF_OK && st != EAF_ENONFINITE) return st;
-  double cont = 0.0;
-  EAF_CUDA(cudaMemcpy(&cont, eaf::assembly_result(h->asm_s, h->nr, h->nth, h->nz),
-                      sizeof(double), cudaMemcpyDeviceToHost));
+  const double cont = h->res_h[1].residual;
   *residual = *cg_res != *cg_res ? *cg_res : cont;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, h->step_ev[0], h->step_ev[1]) == cudaSuccess)
@@ -484,7 +479,7 @@ int eaf_pressure_assemble_f64_device(eaf_cg_t h, const eaf_assembly_fields_t* f,
   int rc = run_assemble(h, d);
   if (rc != EAF_OK) return rc;
   EAF_CUDA(cudaStreamSynchronize(h->st));
-  *residual = h->res_h->residual;
+  *residual = h->res_h[1].residual;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, h->ev[2], h->ev[3]) == cudaSuccess) h->last_kernel_ms = ms;
   return EAF_OK;
@@ -503,7 +498,7 @@ int eaf_pressure_assemble_f64(eaf_cg_t h, const eaf_assembly_fields_t* f, double
   if (rc != EAF_OK) return rc;
   EAF_CUDA(cudaEventRecord(h->ev[5], h->st));
   EAF_CUDA(cudaStreamSynchronize(h->st));
-  *residual = h->res_h->residual;
+  *residual = h->res_h[1].residual;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, h->ev[2], h->ev[3]) == cudaSuccess) h->last_kernel_ms = ms;
   if (cudaEventElapsedTime(&ms, h->ev[0], h->ev[5]) == cudaSuccess) h->last_e2e_ms = ms;

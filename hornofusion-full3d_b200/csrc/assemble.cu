@@ -502,15 +502,15 @@ unsigned asm_grid(long long work) {
 
 }  // namespace
 
-// Scratch: 4 gradient arrays, 12 face arrays (6 per phase), the open bits,
-// the block partials and the residual.
+// Scratch: 4 gradient arrays, 12 face arrays (6 per phase), the open bits and
+// the block partials.
 size_t assembly_scratch_doubles(int nr, int nth, int nz) {
   const size_t nh = (size_t)(nr + 4) * (nth + 4) * (nz + 4);
-  return 16 * nh + (nh + 7) / 8 + 2 * 148 * 8 + 1;
+  return 16 * nh + (nh + 7) / 8 + 2 * 148 * 8;
 }
 
 cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth, int nz,
-                                double* scratch, cudaStream_t st) {
+                                double* scratch, double* result, cudaStream_t st) {
   AsmArgs a;
   a.f = f;
   a.nr = nr;
@@ -537,7 +537,7 @@ cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth,
   a.open = reinterpret_cast<unsigned char*>(take((a.nh + 7) / 8));
   const unsigned gf = asm_grid(a.nh);
   a.part = take(2 * gf);
-  a.result = take(1);
+  a.result = result;
   const bool gi = f.gas_in_poisson != 0, gc = f.gas_compressibility != 0,
              rm = f.liq_room_valid != 0;
   if (gi) asm_gradient_kernel<true><<<gf, kAsmBlock, 0, st>>>(a);
@@ -557,11 +557,6 @@ cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth,
   if (e != cudaSuccess) return e;
   asm_residual_kernel<<<1, kAsmResBlock, 0, st>>>(a, (int)gf);
   return cudaGetLastError();
-}
-
-const double* assembly_result(double* scratch, int nr, int nth, int nz) {
-  const size_t nh = (size_t)(nr + 4) * (nth + 4) * (nz + 4);
-  return scratch + 16 * nh + (nh + 7) / 8 + 2 * (size_t)asm_grid((long long)nh);
 }
 
 }  // namespace eaf

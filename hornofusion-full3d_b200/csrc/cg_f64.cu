@@ -799,6 +799,19 @@ __global__ void fill_marker_kernel(double* p, int n) {
     p[i] = marker;
 }
 
+// All that the waits of a persistent launch look at: the barrier counter (if
+// it has one), the error word, the marked slots.
+__global__ void solver_init_kernel(unsigned long long* counter, int* err, double* slots,
+                                   int nslots) {
+  const double marker = __longlong_as_double((long long)kSlotMarker);
+  const int at = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int i = at; i < nslots; i += gridDim.x * blockDim.x) slots[i] = marker;
+  if (at == 0) {
+    if (counter) *counter = 0;
+    *err = 0;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Single-reduction form (Chronopoulos and Gear, J. Comput. Appl. Math. 25,
 // 1989): the same preconditioned CG with its recurrences rearranged so that an
@@ -1204,12 +1217,21 @@ cudaError_t launch_allreduce_selftest(const GroupWs& ws, uint64_t timeout_ns, in
                                      dim3(mode == 0 ? 2 : 1), dim3(64), args, 0, st);
 }
 
-// The two p.q slot sets of a flat launch of `grid` blocks, filled with the
-// empty-slot marker (group_allsum_slots).
-static cudaError_t fill_pq_slots(const GroupWs& ws, int grid, cudaStream_t st) {
-  // (harmless where the kernel keeps the counter form for p.q)
-  if (grid <= 1 || grid > 32 * kPerLane) return cudaSuccess;
-  fill_marker_kernel<<<1, 320, 0, st>>>(ws.part + (size_t)kPqSlotOffset * grid, 2 * grid);
+// The counter and the error word of a persistent launch.
+cudaError_t launch_group_init(const GroupWs& ws, cudaStream_t st) {
+  (void)cudaGetLastError();  // report this launch's error, not an older one
+  solver_init_kernel<<<1, 32, 0, st>>>(ws.counter, ws.err, nullptr, 0);
+  return cudaGetLastError();
+}
+// Before a flat launch of `grid` blocks: the counter, the error word and the
+// two p.q slot sets (group_allsum_slots), in one launch where two memsets and
+// a fill took 4 us more.
+static cudaError_t init_flat(const GroupWs& ws, int grid, cudaStream_t st) {
+  (void)cudaGetLastError();  // report this launch's error, not an older one
+  // (the slots are harmless where the kernel keeps the counter form for p.q)
+  const int nslots = grid <= 1 || grid > 32 * kPerLane ? 0 : 2 * grid;
+  solver_init_kernel<<<1, 320, 0, st>>>(ws.counter, ws.err, ws.part + (size_t)kPqSlotOffset * grid,
+                                        nslots);
   return cudaGetLastError();
 }
 
@@ -1233,9 +1255,7 @@ cudaError_t launch_cg_f64(const MeshDims& d, const SysF64& s, const GroupWs& ws,
   a.max_iter = max_iter;
   a.tol = tol;
   a.timeout_ns = timeout_ns;
-  cudaError_t e = cudaMemsetAsync(ws.counter, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
-  if (e == cudaSuccess) e = fill_pq_slots(ws, grid, st);
+  cudaError_t e = init_flat(ws, grid, st);
   if (e != cudaSuccess) return e;
   const void* k = cg_f64_kernel_ptr(block, d.n);
   void* args[] = {&a};
@@ -1341,9 +1361,8 @@ cudaError_t launch_cg_f64_cluster(const MeshDims& d, const SysF64& s, const Grou
   if (e != cudaSuccess) return e;
   (void)cudaGetLastError();  // report this launch's error, not an older one
   const int nslots = (int)cluster_slot_doubles(grid / cluster);
-  fill_marker_kernel<<<(nslots + 255) / 256, 256, 0, st>>>(slots, nslots);
+  solver_init_kernel<<<(nslots + 255) / 256, 256, 0, st>>>(nullptr, ws.err, slots, nslots);
   e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   void* args[] = {&a, &slots};
   cudaLaunchAttribute attr[2];
@@ -1477,9 +1496,7 @@ cudaError_t launch_cg_f64_keep(const MeshDims& d, const SysF64& s, const GroupWs
   std::lock_guard<std::mutex> attr_lock(launch_attr_mutex());
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.counter, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
-  if (e == cudaSuccess) e = fill_pq_slots(ws, grid, st);
+  if (e == cudaSuccess) e = init_flat(ws, grid, st);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(block), args, smem, st);

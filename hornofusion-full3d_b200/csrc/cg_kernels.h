@@ -71,6 +71,9 @@ struct GroupWs {
 MeshDims make_dims(int nr, int nth, int nz);
 
 
+// Zeroes the counter and the error word of a persistent launch.
+cudaError_t launch_group_init(const GroupWs& ws, cudaStream_t st);
+
 // pack: halo layout -> compact layout, symmetry check, FP64 initial
 // residual r = Su - A phi with the reference stencil (phi's theta halo
 // wrapped, its r/z halo cells read as given).
@@ -248,12 +251,11 @@ cudaError_t launch_pcorr_f64(const eaf_pcorr_fields_t& f, int nr, int nth, int n
 
 // Pressure-equation assembly (solve_pressure_correction before the CG), three
 // launches on `st` into device pointers of `f`; `scratch` holds
-// assembly_scratch_doubles() doubles (gradients, block partials, and the
-// residual at assembly_result()).
+// assembly_scratch_doubles() doubles (gradients, faces, block partials), the
+// residual goes to `result` (the device address of pinned memory, or device memory).
 size_t assembly_scratch_doubles(int nr, int nth, int nz);
 cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth, int nz,
-                                double* scratch, cudaStream_t st);
-const double* assembly_result(double* scratch, int nr, int nth, int nz);
+                                double* scratch, double* result, cudaStream_t st);
 
 // Threads per block of the batched kernels (FP64 and mixed).
 constexpr int kBatchBlock = 512;

@@ -20,7 +20,7 @@ struct eaf_cg {
   eaf::SysF32 f;
   bool have_f32;
   eaf::GroupWs ws;
-  eaf::SolveResult* res_h;  // pinned
+  eaf::SolveResult* res_h;  // pinned, two: a solve's, the assembly's; ws.result on the device
   int block, grid;     // 0 = automatic
   int cluster;         // blocks per thread-block cluster; 0 = automatic, 1 = none
   int resident;        // one-cluster launches keep the system in shared memory
@@ -35,7 +35,7 @@ struct eaf_cg {
   int last_sym, last_kernels;
   int last_grid, last_block, last_cluster;
   double* tdma_mbox;  // TDMA line hand-over slots (lazy)
-  double* tdma_fac;  // TDMA line factors (lazy)
+  double* tdma_fac;   // TDMA line records, behind them
   double* pc_d;      // post-CG correction mirror: doubles (lazy)
   int* pc_i;         // post-CG correction mirror: ints (lazy)
   int form;          // EAF_CG_FORM_*: the FP64 solver's recurrences

@@ -1271,8 +1271,7 @@ cudaError_t launch_residual_f64(const HaloInputs& in, const double* phi, const M
   a.sxy = (long long)(d.nr + 4) * (d.nth + 4);
   a.ws = ws;
   a.timeout_ns = timeout_ns;
-  cudaError_t e = cudaMemsetAsync(ws.counter, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
+  const cudaError_t e = launch_group_init(ws, st);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel((const void*)residual_kernel, dim3(grid), dim3(kResBlock),
