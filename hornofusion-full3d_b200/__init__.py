@@ -135,30 +135,25 @@ class CGSolver:
         ``fields`` (an object with the attributes of eafgen.PcorrFields:
         float64 halo-layout arrays, int32 flag/mask arrays, coordinate
         arrays, ``has_gas``, ``alpha_p``)."""
-        from ._lib import PcorrFieldsC, PhaseFields
-
-        def addr(a, kind):
-            if isinstance(a, np.ndarray):
-                want = np.float64 if kind == "d" else np.int32
-                if a.dtype != want or not a.flags.c_contiguous:
-                    raise ValueError(f"array must be C-contiguous {np.dtype(want)}")
-                return a.ctypes.data
-            if hasattr(a, "data_ptr"):
-                return a.data_ptr()
-            raise TypeError(f"unsupported array type {type(a)!r}")
+        from ._lib import PCORR_LAYOUT, PCORR_NAMES, PcorrFieldsC
 
         c = PcorrFieldsC()
-        for n in ("pp", "Fs_r", "Fs_th", "Fs_z", "ac_r", "ac_th", "ac_z", "Fc_r", "Fc_th",
-                  "Fc_z", "vol", "r", "theta", "z", "p"):
-            setattr(c, n, addr(getattr(fields, n), "d"))
-        for n in ("lk_r", "lk_th", "lk_z", "cell_type", "act_l", "act_g"):
-            setattr(c, n, addr(getattr(fields, n), "i"))
-        for ph in ("liq", "gas") if fields.has_gas else ("liq",):
-            pf = PhaseFields(*[addr(getattr(fields, ph + "_" + n), "d") for n in
-                               ("alpha", "aP_ur", "aP_uth", "aP_uz", "ur", "uth", "uz")])
-            setattr(c, ph, pf)
-        c.has_gas = 1 if fields.has_gas else 0
-        c.alpha_p = float(fields.alpha_p)
+        ptrs = []
+        for names, want, phase in PCORR_NAMES:
+            if phase == "gas" and not fields.has_gas:
+                ptrs += [0] * len(names)
+                continue
+            for n in names:
+                a = getattr(fields, n)
+                if isinstance(a, np.ndarray):
+                    if a.dtype != want or not a.flags.c_contiguous:
+                        raise ValueError(f"array must be C-contiguous {np.dtype(want)}")
+                    ptrs.append(a.ctypes.data)
+                elif hasattr(a, "data_ptr"):
+                    ptrs.append(a.data_ptr())
+                else:
+                    raise TypeError(f"unsupported array type {type(a)!r}")
+        PCORR_LAYOUT.pack_into(c, 0, *ptrs, 1 if fields.has_gas else 0, float(fields.alpha_p))
         fn = (self._lib.eaf_pressure_correct_f64_device if device_ptrs
               else self._lib.eaf_pressure_correct_f64)
         check(fn(self._h, ctypes.byref(c)), "eaf_pressure_correct_f64")
@@ -166,35 +161,27 @@ class CGSolver:
     def _assembly_struct(self, fields):
         """eaf_assembly_fields_t of ``fields`` (numpy arrays or device
         tensors; attributes the switches leave unread may be None)."""
-        from ._lib import ASSEMBLY_IN, ASSEMBLY_OUT, AssemblyFieldsC, PhaseState
+        from ._lib import ASSEMBLY_INS, ASSEMBLY_LAYOUT, ASSEMBLY_NAMES, AssemblyFieldsC
 
-        ints = ("cell_type", "outlet", "act_l", "act_g", "lk_r", "lk_th", "lk_z")
-
-        def addr(name, a):
+        ptrs = []
+        for name, want in ASSEMBLY_NAMES:
+            a = getattr(fields, name, None)
             if a is None:
-                return None
-            if isinstance(a, np.ndarray):
-                want = np.int32 if name in ints else np.float64
+                ptrs.append(0)
+            elif isinstance(a, np.ndarray):
                 if a.dtype != want or not a.flags.c_contiguous:
                     raise ValueError(f"{name} must be C-contiguous {np.dtype(want)}")
-                return a.ctypes.data
-            if hasattr(a, "data_ptr"):
-                return a.data_ptr()
-            raise TypeError(f"unsupported array type {type(a)!r}")
-
-        c = AssemblyFieldsC()
-        for n in ASSEMBLY_IN + ASSEMBLY_OUT:
-            setattr(c, n, addr(n, getattr(fields, n, None)))
-        for ph in ("liq", "gas"):
-            setattr(c, ph, PhaseState(*[addr(n, getattr(fields, ph + "_" + n, None)) for n in
-                                        ("alpha", "rho", "ur", "uth", "uz", "aP_ur",
-                                         "aP_uth", "aP_uz")]))
-        c.liq_T = addr("liq_T", getattr(fields, "liq_T", None))
-        c.gas_T_old = addr("gas_T_old", getattr(fields, "gas_T_old", None))
+                ptrs.append(a.ctypes.data)
+            elif hasattr(a, "data_ptr"):
+                ptrs.append(a.data_ptr())
+            else:
+                raise TypeError(f"unsupported array type {type(a)!r}")
         fl = int(fields.flags)
-        c.liq_room_valid, c.gas_in_poisson, c.gas_compressibility = \
-            fl & 1, (fl >> 1) & 1, (fl >> 2) & 1
-        c.dt, c.rho_gas, c.T_ambient, c.beta_expansion = [float(x) for x in fields.scalars]
+        c = AssemblyFieldsC()
+        dt, rho_gas, T_ambient, beta_expansion = [float(x) for x in fields.scalars]
+        ASSEMBLY_LAYOUT.pack_into(c, 0, *ptrs[:ASSEMBLY_INS], fl & 1, (fl >> 1) & 1,
+                                  (fl >> 2) & 1, dt, rho_gas, T_ambient, beta_expansion,
+                                  *ptrs[ASSEMBLY_INS:])
         return c
 
     def pressure_assemble(self, fields, device_ptrs: bool = False) -> float:
