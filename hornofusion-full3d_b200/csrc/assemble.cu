@@ -5,7 +5,11 @@
 //      gas, the vertical one with the liquid weight (gas_gz :421-440; its r
 //      and theta gradients equal the liquid's); one thread per halo element,
 //      theta halo rows computing their source row of the periodic copy, so
-//      neither a clearing pass nor a halo pass is needed;
+//      neither a clearing pass nor a halo pass is needed. A second row of
+//      blocks forms, per phase and component, the quotient alpha vol /
+//      max(aP, SMALL) of every element: d_f of a face is the mean of two of
+//      them, so each serves two faces, and the face pass (bound by the
+//      instructions of 12 FP64 divisions an element) makes none of its own;
 //   F. faces: add_phase_contribution (:469-619) evaluates every interior
 //      face twice, once from each side, and both evaluations are the same
 //      arithmetic (the two-term sums commute exactly); so each face is
@@ -61,7 +65,9 @@ struct AsmArgs {
   double* part;                    // [2][grid] block partials
   double* result;                  // residual
   int nr, nth, nz;
+  double *dl[3], *dg[3];           // alpha vol / max(aP, SMALL) per component, liquid and gas
   unsigned sx, sxy, rows, nh;      // halo strides, theta rows, elements
+  FastDiv fd_sx, fd_rows;
 };
 
 template <typename T>
@@ -98,11 +104,22 @@ __device__ __forceinline__ double liq_weight(double beta, double ta, bool la, do
 
 // Halo element q -> (i, j, k), 1-based interior indices.
 __device__ __forceinline__ void cell_of(const AsmArgs& a, unsigned q, int& i, int& j, int& k) {
-  const unsigned u = q / a.sx;
+  const unsigned u = a.fd_sx.div(q);
   i = (int)(q - u * a.sx) - 1;
-  const unsigned v = u / a.rows;
+  const unsigned v = a.fd_rows.div(u);
   j = (int)(u - v * a.rows) - 1;
   k = (int)v - 1;
+}
+
+// The three quotients alpha vol / max(aP, SMALL) of one phase at element q,
+// each a term of d_f for two faces.
+__device__ __forceinline__ void cell_quotients(const eaf_phase_state_t& ph, double vol, unsigned q,
+                                               double* const* out) {
+  const double t = ld(ph.alpha, q) * vol;
+  const double a0 = ld(ph.aP_ur, q), a1 = ld(ph.aP_uth, q), a2 = ld(ph.aP_uz, q);
+  out[0][q] = t / fmax(a0, kS);
+  out[1][q] = t / fmax(a1, kS);
+  out[2][q] = t / fmax(a2, kS);
 }
 
 // Every load of a cell is issued before the first decision that depends on
@@ -111,6 +128,15 @@ __device__ __forceinline__ void cell_of(const AsmArgs& a, unsigned q, int& i, in
 template <bool GAS_IN>
 __global__ void __launch_bounds__(kAsmBlock, 4) asm_gradient_kernel(AsmArgs a) {
   const eaf_assembly_fields_t& f = a.f;
+  if (blockIdx.y == 1) {
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < a.nh;
+         q += gridDim.x * blockDim.x) {
+      const double vol = ld(f.vol, q);
+      cell_quotients(f.liq, vol, q, a.dl);
+      if (GAS_IN) cell_quotients(f.gas, vol, q, a.dg);
+    }
+    return;
+  }
   for (unsigned qd = blockIdx.x * blockDim.x + threadIdx.x; qd < a.nh;
        qd += gridDim.x * blockDim.x) {
     int i, jd, k;
@@ -196,7 +222,7 @@ __device__ __forceinline__ bool face_open(double u_f, double room_neg, double ro
 struct LowerFaces {
   unsigned q, x[3];
   int ct[4];  // q, w, s, b
-  double p[4], vol[4], room[4];
+  double p[4], room[4];
   double delta[3], y[3], gp[3], area[3];
   bool ok[3];
 };
@@ -207,23 +233,22 @@ struct LowerFaces {
 template <bool ISG, bool ROOM>
 __device__ __forceinline__ unsigned phase_faces(const AsmArgs& a, const LowerFaces& L,
                                                 const eaf_phase_state_t& ph, const int* act,
-                                                const double* gz, double lw_b,
+                                                const double* gz, double* const* dq, double lw_b,
                                                 const FacePhase& out) {
   const unsigned q = L.q;
   const int ac_q = ld(act, q);
   const double al_q = ld(ph.alpha, q);
-  const double* apd[3] = {ph.aP_ur, ph.aP_uth, ph.aP_uz};
   const double* ud[3] = {ph.ur, ph.uth, ph.uz};
   const double* gd[3] = {a.gr, a.gth, gz};
   int ac_x[3];
-  double al_x[3], ap_q[3], ap_x[3], u_q[3], u_x[3], g_q[3], g_x[3];
+  double al_x[3], d_q[3], d_x[3], u_q[3], u_x[3], g_q[3], g_x[3];
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
     const unsigned x = L.x[f];
     ac_x[f] = ld(act, x);
     al_x[f] = ld(ph.alpha, x);
-    ap_q[f] = ld(apd[f], q);
-    ap_x[f] = ld(apd[f], x);
+    d_q[f] = dq[f][q];
+    d_x[f] = dq[f][x];
     u_q[f] = ld(ud[f], q);
     u_x[f] = ld(ud[f], x);
     g_q[f] = ld(gd[f], q);
@@ -234,8 +259,7 @@ __device__ __forceinline__ unsigned phase_faces(const AsmArgs& a, const LowerFac
   double af[3], d_f[3], u_f[3];
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
-    d_f[f] = 0.5 * (al_q * L.vol[0] / fmax(ap_q[f], kS) +
-                    al_x[f] * L.vol[f + 1] / fmax(ap_x[f], kS));
+    d_f[f] = 0.5 * (d_q[f] + d_x[f]);
     af[f] = 0.5 * (al_q + al_x[f]);
     u_f[f] = 0.5 * (u_q[f] + u_x[f]) + d_f[f] * (0.5 * (g_q[f] + g_x[f]) - L.gp[f] - lw[f]);
     const bool link = (L.ct[0] != 0) & (ac_q != 0) & (L.ct[f + 1] != 0) & (ac_x[f] != 0);
@@ -252,8 +276,11 @@ __device__ __forceinline__ unsigned phase_faces(const AsmArgs& a, const LowerFac
 
 // One thread per halo element whose lower faces some interior cell adds:
 // i in 1..nr+1, j in 1..nth+1, k in 1..nz+1 (the others are never read).
+// 60x120x84, us with caches cold: 84 with its own quotients (G then 23), 46
+// with G's (G 41), 42 in 80 registers, three blocks an SM. (A thread a phase:
+// 84, 95 in 80 registers. The cell pass in 80 registers spills: 49 for 44.)
 template <bool GAS_IN, bool ROOM>
-__global__ void __launch_bounds__(kAsmBlock, 2) asm_face_kernel(AsmArgs a) {
+__global__ void __launch_bounds__(kAsmBlock, 3) asm_face_kernel(AsmArgs a) {
   const eaf_assembly_fields_t& f = a.f;
   for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < a.nh;
        q += gridDim.x * blockDim.x) {
@@ -270,7 +297,6 @@ __global__ void __launch_bounds__(kAsmBlock, 2) asm_face_kernel(AsmArgs a) {
     for (int m = 0; m < 4; ++m) {
       L.ct[m] = ld(f.cell_type, cell[m]);
       L.p[m] = ld(f.p, cell[m]);
-      L.vol[m] = ld(f.vol, cell[m]);
       L.room[m] = ROOM ? ld(f.liq_room, cell[m]) : 1.0;
     }
     const double r0 = ld(f.r, i), r1 = ld(f.r, i + 1);
@@ -289,7 +315,7 @@ __global__ void __launch_bounds__(kAsmBlock, 2) asm_face_kernel(AsmArgs a) {
       // + side minus - side
       L.gp[m] = div_by_recip(L.p[0] - L.p[m + 1], L.delta[m], L.y[m], L.ok[m]);
     }
-    unsigned bits = phase_faces<false, ROOM>(a, L, f.liq, f.act_l, a.gz_l, 0.0, a.fl);
+    unsigned bits = phase_faces<false, ROOM>(a, L, f.liq, f.act_l, a.gz_l, a.dl, 0.0, a.fl);
     if (GAS_IN) {
       // liquid weight of the B face (liq_weight_f :407-417, lower cell first)
       const unsigned b = L.x[2];
@@ -297,7 +323,7 @@ __global__ void __launch_bounds__(kAsmBlock, 2) asm_face_kernel(AsmArgs a) {
                                      ld(f.liq.alpha, b), ld(f.liq.rho, b), ld(f.liq_T, b),
                                      ld(f.act_l, q) != 0, ld(f.liq.alpha, q),
                                      ld(f.liq.rho, q), ld(f.liq_T, q));
-      bits |= phase_faces<true, false>(a, L, f.gas, f.act_g, a.gz_g, lw_b, a.fg) << kGasShift;
+      bits |= phase_faces<true, false>(a, L, f.gas, f.act_g, a.gz_g, a.dg, lw_b, a.fg) << kGasShift;
     }
     a.open[q] = (unsigned char)bits;
   }
@@ -502,11 +528,11 @@ unsigned asm_grid(long long work) {
 
 }  // namespace
 
-// Scratch: 4 gradient arrays, 12 face arrays (6 per phase), the open bits and
-// the block partials.
+// Scratch: 4 gradient arrays, 12 face arrays (6 per phase), 6 of quotients, the
+// open bits and the block partials.
 size_t assembly_scratch_doubles(int nr, int nth, int nz) {
   const size_t nh = (size_t)(nr + 4) * (nth + 4) * (nz + 4);
-  return 16 * nh + (nh + 7) / 8 + 2 * 148 * 8;
+  return 22 * nh + (nh + 7) / 8 + 2 * 148 * 8;
 }
 
 cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth, int nz,
@@ -534,14 +560,20 @@ cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth,
     F->cB = take(a.nh);
     F->fB = take(a.nh);
   }
+  for (int m = 0; m < 3; ++m) {
+    a.dl[m] = take(a.nh);
+    a.dg[m] = take(a.nh);
+  }
   a.open = reinterpret_cast<unsigned char*>(take((a.nh + 7) / 8));
+  a.fd_sx = FastDiv(a.sx);
+  a.fd_rows = FastDiv(a.rows);
   const unsigned gf = asm_grid(a.nh);
   a.part = take(2 * gf);
   a.result = result;
   const bool gi = f.gas_in_poisson != 0, gc = f.gas_compressibility != 0,
              rm = f.liq_room_valid != 0;
-  if (gi) asm_gradient_kernel<true><<<gf, kAsmBlock, 0, st>>>(a);
-  else asm_gradient_kernel<false><<<gf, kAsmBlock, 0, st>>>(a);
+  if (gi) asm_gradient_kernel<true><<<dim3(gf, 2), kAsmBlock, 0, st>>>(a);
+  else asm_gradient_kernel<false><<<dim3(gf, 2), kAsmBlock, 0, st>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   using K = void (*)(AsmArgs);

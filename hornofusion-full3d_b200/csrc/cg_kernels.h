@@ -251,7 +251,7 @@ cudaError_t launch_pcorr_f64(const eaf_pcorr_fields_t& f, int nr, int nth, int n
 
 // Pressure-equation assembly (solve_pressure_correction before the CG), three
 // launches on `st` into device pointers of `f`; `scratch` holds
-// assembly_scratch_doubles() doubles (gradients, faces, block partials), the
+// assembly_scratch_doubles() doubles (gradients, quotients, faces, block partials), the
 // residual goes to `result` (the device address of pinned memory, or device memory).
 size_t assembly_scratch_doubles(int nr, int nth, int nz);
 cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth, int nz,
