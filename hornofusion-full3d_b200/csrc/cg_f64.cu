@@ -1056,11 +1056,11 @@ struct PackArgs {
   long long hy, hz;  // halo strides of j and k
 };
 
-__global__ void pack_f64_kernel(PackArgs a) {
+// Block `block` of `blocks` that share one system.
+__device__ __forceinline__ void pack_cells(const PackArgs& a, int block, int blocks) {
   const MeshDims& d = a.d;
   const HaloInputs& in = a.in;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d.n;
-       c += gridDim.x * blockDim.x) {
+  for (int c = block * blockDim.x + threadIdx.x; c < d.n; c += blocks * blockDim.x) {
     int i, j, k;
     cell_ijk(d, c, i, j, k);
     const long long h = (long long)(i + 2) + a.hy * (j + 2) + a.hz * (k + 2);
@@ -1116,10 +1116,10 @@ __device__ __forceinline__ int theta_source(int j, int nth) {
   return 2 <= nth ? 2 : 1;  // j == nth + 2
 }
 
-__global__ void unpack_f64_kernel(UnpackArgs a) {
+__device__ __forceinline__ void unpack_cells(const UnpackArgs& a, int block, int blocks) {
   const MeshDims& d = a.d;
-  for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < a.total;
-       h += (long long)gridDim.x * blockDim.x) {
+  for (long long h = block * (long long)blockDim.x + threadIdx.x; h < a.total;
+       h += (long long)blocks * blockDim.x) {
     // halo coordinates -> Fortran indices
     const uint32_t t = a.fd_hy.div((uint32_t)h);
     const int i = (int)(h - (long long)t * a.hy) - 1;
@@ -1140,28 +1140,43 @@ __global__ void unpack_f64_kernel(UnpackArgs a) {
   }
 }
 
-}  // namespace
+__global__ void pack_f64_kernel(PackArgs a) { pack_cells(a, blockIdx.x, gridDim.x); }
+__global__ void unpack_f64_kernel(UnpackArgs a) { unpack_cells(a, blockIdx.x, gridDim.x); }
 
-cudaError_t launch_pack_f64(const MeshDims& d, const HaloInputs& in, const SysF64& s,
-                            cudaStream_t st) {
+// The same for many systems in one launch: `map` gives each block its system
+// (x), its index (y) and the number of blocks (z) among that system's.
+struct IoRow {
+  PackArgs pack;
+  UnpackArgs unpack;
+};
+__global__ void pack_many_kernel(const IoRow* rows, const int4* map) {
+  const int4 m = map[blockIdx.x];
+  const PackArgs a = rows[m.x].pack;
+  pack_cells(a, m.y, m.z);
+}
+__global__ void unpack_many_kernel(const IoRow* rows, const int4* map) {
+  const int4 m = map[blockIdx.x];
+  const UnpackArgs a = rows[m.x].unpack;
+  unpack_cells(a, m.y, m.z);
+}
+
+constexpr int kIoBlock = 256;
+int io_blocks(long long work) {
+  const long long g = (work + kIoBlock - 1) / kIoBlock;
+  return (int)(g > 148 * 16 ? 148 * 16 : g);
+}
+
+PackArgs pack_args(const MeshDims& d, const HaloInputs& in, const SysF64& s) {
   PackArgs a;
   a.d = d;
   a.in = in;
   a.s = s;
   a.hy = d.nr + 4;
   a.hz = (long long)(d.nr + 4) * (d.nth + 4);
-  (void)cudaGetLastError();  // report this launch's error, not an older one
-  cudaError_t e = cudaMemsetAsync(s.asym, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  const int block = 256;
-  int grid = (d.n + block - 1) / block;
-  if (grid > 148 * 16) grid = 148 * 16;
-  pack_f64_kernel<<<grid, block, 0, st>>>(a);
-  return cudaGetLastError();
+  return a;
 }
 
-cudaError_t launch_unpack_f64(const MeshDims& d, const double* x, double* phi,
-                              cudaStream_t st) {
+UnpackArgs unpack_args(const MeshDims& d, const double* x, double* phi) {
   UnpackArgs a;
   a.d = d;
   a.x = x;
@@ -1171,11 +1186,48 @@ cudaError_t launch_unpack_f64(const MeshDims& d, const double* x, double* phi,
   a.fd_hy = FastDiv((uint32_t)a.hy);
   a.fd_hj = FastDiv((uint32_t)a.hj);
   a.total = (long long)(d.nr + 4) * (d.nth + 4) * (d.nz + 4);
+  return a;
+}
+
+}  // namespace
+
+cudaError_t launch_pack_f64(const MeshDims& d, const HaloInputs& in, const SysF64& s,
+                            cudaStream_t st) {
   (void)cudaGetLastError();  // report this launch's error, not an older one
-  const int block = 256;
-  long long g = (a.total + block - 1) / block;
-  int grid = (int)(g > 148 * 16 ? 148 * 16 : g);
-  unpack_f64_kernel<<<grid, block, 0, st>>>(a);
+  cudaError_t e = cudaMemsetAsync(s.asym, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  pack_f64_kernel<<<io_blocks(d.n), kIoBlock, 0, st>>>(pack_args(d, in, s));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_unpack_f64(const MeshDims& d, const double* x, double* phi,
+                              cudaStream_t st) {
+  (void)cudaGetLastError();  // report this launch's error, not an older one
+  const UnpackArgs a = unpack_args(d, x, phi);
+  unpack_f64_kernel<<<io_blocks(a.total), kIoBlock, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+size_t io_row_bytes() { return sizeof(IoRow); }
+
+void fill_io_row(void* row, int id, const MeshDims& d, const HaloInputs& in, const SysF64& s,
+                 double* phi, std::vector<int4>* map) {
+  IoRow* r = static_cast<IoRow*>(row);
+  r->pack = pack_args(d, in, s);
+  r->unpack = unpack_args(d, s.x, phi);
+  const int blocks = io_blocks(d.n);
+  for (int b = 0; b < blocks; ++b) map->push_back(make_int4(id, b, blocks, 0));
+}
+
+cudaError_t launch_pack_many(const void* rows, const int4* map, int blocks, cudaStream_t st) {
+  (void)cudaGetLastError();  // report this launch's error, not an older one
+  pack_many_kernel<<<blocks, kIoBlock, 0, st>>>(static_cast<const IoRow*>(rows), map);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_unpack_many(const void* rows, const int4* map, int blocks, cudaStream_t st) {
+  (void)cudaGetLastError();  // report this launch's error, not an older one
+  unpack_many_kernel<<<blocks, kIoBlock, 0, st>>>(static_cast<const IoRow*>(rows), map);
   return cudaGetLastError();
 }
 

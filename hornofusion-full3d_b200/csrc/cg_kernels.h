@@ -3,6 +3,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <vector>
 #include <stdint.h>
 
 #include <mutex>
@@ -70,6 +72,15 @@ struct GroupWs {
 
 MeshDims make_dims(int nr, int nth, int nz);
 
+
+// Pack and unpack of many systems, each in one launch over a device table of
+// rows (io_row_bytes() each) and a device map of blocks, which fill_io_row
+// appends to; the symmetry flags must be zero before the pack.
+size_t io_row_bytes();
+void fill_io_row(void* row, int id, const MeshDims& d, const HaloInputs& in, const SysF64& s,
+                 double* phi, std::vector<int4>* map);
+cudaError_t launch_pack_many(const void* rows, const int4* map, int blocks, cudaStream_t st);
+cudaError_t launch_unpack_many(const void* rows, const int4* map, int blocks, cudaStream_t st);
 
 // Zeroes the counter and the error word of a persistent launch.
 cudaError_t launch_group_init(const GroupWs& ws, cudaStream_t st);
