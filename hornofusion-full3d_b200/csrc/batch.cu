@@ -236,6 +236,14 @@ struct eaf_batch {
 
 namespace {
 
+// Uploads a table from pageable memory on the batch's stream, which is
+// non-blocking: nothing orders it behind a copy on the default stream, and such
+// a copy may return before its transfer has landed. The source may go
+// once the stream has been synchronised.
+cudaError_t upload(const eaf_batch* b, void* to, const void* from, size_t bytes) {
+  return cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, b->st);
+}
+
 int width_for(const eaf_batch* b, int s) {
   if (b->width[s] > 0) return b->width[s];
   return eaf::tuned_lane_width(b->nr[s], b->nth[s], b->nz[s]);
@@ -286,8 +294,8 @@ int alloc_f32(eaf_batch* b) {
       }
     }
   }
-  cudaError_t e = cudaMemcpy(b->d_sys, b->sys.data(), sizeof(BatchSys) * b->nsys,
-                             cudaMemcpyHostToDevice);
+  cudaError_t e = upload(b, b->d_sys, b->sys.data(), sizeof(BatchSys) * b->nsys);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
   if (e != cudaSuccess) {
     eaf::set_error("eaf_batch: table upload", e);
     return EAF_ECUDA;
@@ -343,13 +351,14 @@ int plan(eaf_batch* b) {
   b->d_counters = nullptr;
   b->d_parts = nullptr;
   cudaError_t e = cudaMalloc((void**)&b->d_tab, sizeof(int) * host.size());
-  if (e == cudaSuccess)
-    e = cudaMemcpy(b->d_tab, host.data(), sizeof(int) * host.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(b, b->d_tab, host.data(), sizeof(int) * host.size());
   if (e == cudaSuccess)
     e = cudaMalloc((void**)&b->d_counters,
                    sizeof(unsigned long long) * eaf::kCounterStride *
                        (b->nlanes > 0 ? b->nlanes : 1));
   if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_parts, sizeof(double) * 8 * (G > 0 ? G : 1));
+  const cudaError_t sync = cudaStreamSynchronize(b->st);  // (`host` goes)
+  if (e == cudaSuccess) e = sync;
   if (e != cudaSuccess) {
     eaf::set_error("eaf_batch: plan tables", e);
     return EAF_ENOMEM;
@@ -425,9 +434,10 @@ cudaError_t upload_io(eaf_batch* b) {
   if (!b->d_io) e = cudaMalloc(&b->d_io, rows.size());
   if (e == cudaSuccess && !b->d_io_map)
     e = cudaMalloc((void**)&b->d_io_map, sizeof(int4) * map.size());
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_io, rows.data(), rows.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(b->d_io_map, map.data(), sizeof(int4) * map.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(b, b->d_io, rows.data(), rows.size());
+  if (e == cudaSuccess) e = upload(b, b->d_io_map, map.data(), sizeof(int4) * map.size());
+  const cudaError_t sync = cudaStreamSynchronize(b->st);  // (`rows` and `map` go)
+  if (e == cudaSuccess) e = sync;
   b->io_blocks = (int)map.size();
   // Systems whose phi overlap are unpacked one after another: the last one's
   // values stay.
@@ -531,8 +541,8 @@ int eaf_batch_create(eaf_batch_t* out, int nsys, const int* dims, int device) {
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
   for (int s = 0; s < nsys && e == cudaSuccess; ++s) b->sys[s].result = b->d_res + s;
-  if (e == cudaSuccess)
-    e = cudaMemcpy(b->d_sys, b->sys.data(), sizeof(BatchSys) * nsys, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload(b, b->d_sys, b->sys.data(), sizeof(BatchSys) * nsys);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
   if (e != cudaSuccess) {
     eaf::set_error("eaf_batch_create", e);
     free_batch(b);
