@@ -254,6 +254,11 @@ __device__ __forceinline__ void bulk_copy_s2g(double* dst, const double* src, in
                : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// Orders this thread's view of shared memory (generic proxy) before bulk copies
+// (async proxy) that are issued behind it.
+__device__ __forceinline__ void fence_proxy_async() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 __device__ __forceinline__ void bulk_copies_done() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
@@ -356,13 +361,13 @@ __global__ void __launch_bounds__(kTileBlock) tdma_factor_kernel(FactorArgs a) {
       for (int arr = 0; arr < kRArrays; ++arr) r[arr * K] = arr == kRM ? 1.0 : 0.0;
     }
   }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the bulk stores
+  fence_proxy_async();  // before the bulk stores
   __syncthreads();
   for (int u = warp; u < tl.lines; u += kTileBlock / 32) {
     double* rec = sm + (size_t)u * g.rec;
     const int ch = tl.a_of(d, u), b = tl.b_of(d, u);
     factor_line<K>(d, g, rec, lane);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    fence_proxy_async();
     __syncwarp();
     if (lane == 0) bulk_copy_s2g(a.rec + ((long long)b * d.A + ch) * g.rec, rec, g.rec * 8);
     if (b % g.G == 0) {
@@ -405,7 +410,7 @@ __global__ void __launch_bounds__(kTileBlock) tdma_old_kernel(OldArgs a) {
     r[kO2 * K] = o2;
     r[kOEnd * K] = end;
   }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  fence_proxy_async();
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int u = 0; u < tl.lines; ++u)
@@ -581,7 +586,11 @@ __device__ void load_lines(const SweepArgs& a, int w, double* bufs, uint64_t* fu
     } else if (__all_sync(kAllLanes, mbar_look(smem_addr(&empty[done.st]), done.phase))) {
       write_line<K>(a, bufs + (size_t)done.st * g.buf + g.rec + kOScalars + lane * Ln::kOld,
                     done.b, done.ch, lane);
-      __syncwarp();  // every lane has read its values before the buffer is filled again
+      // The solver wrote its values, and the lanes here read them, by the generic
+      // proxy; the copy that fills the buffer again writes by the async one, after
+      // every lane's fence.
+      fence_proxy_async();
+      __syncwarp();
       done.next(d, g);
       --ahead;
       wait = Patience();
