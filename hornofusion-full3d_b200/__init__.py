@@ -561,3 +561,10 @@ def allreduce_timeout_selftest(device: int = 0, timeout_ms: float = 20.0, mode: 
     count never completes; mode 1: a partial is never written) must give
     EAF_ETIMEOUT."""
     return load().eaf_selftest_allreduce_timeout(device, float(timeout_ms), int(mode))
+
+
+def push_timeout_selftest(device: int = 0, timeout_ms: float = 20.0) -> int:
+    """The cluster-resident solver's pushed exchange, entered by one of two
+    blocks only, must give EAF_ETIMEOUT, and both blocks leave after the copies
+    in flight have landed."""
+    return load().eaf_selftest_push_timeout(device, float(timeout_ms))

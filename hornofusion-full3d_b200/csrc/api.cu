@@ -688,9 +688,8 @@ int eaf_selftest_barrier_timeout(int device, double timeout_ms) {
   return err_h;
 }
 
-int eaf_selftest_allreduce_timeout(int device, double timeout_ms, int mode) {
-  if (!(timeout_ms > 0.0) || timeout_ms > 10000.0 || (mode != 0 && mode != 1))
-    return EAF_EINVAL;
+// Modes 0 and 1: the release-free all-reduce's; 2: the pushed exchange's.
+static int run_wait_selftest(int device, double timeout_ms, int mode) {
   eaf::DeviceGuard guard(device);
   if (!guard.ok()) return EAF_ECUDA;
   GroupWs ws = {};
@@ -700,8 +699,10 @@ int eaf_selftest_allreduce_timeout(int device, double timeout_ms, int mode) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&ws.part, sizeof(double) * 16);
   if (e == cudaSuccess) e = cudaMalloc((void**)&ws.counter, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc((void**)&ws.err, sizeof(int));
+  const uint64_t ns = (uint64_t)(timeout_ms * 1.0e6);
   if (e == cudaSuccess)
-    e = eaf::launch_allreduce_selftest(ws, (uint64_t)(timeout_ms * 1.0e6), mode, st);
+    e = mode == 2 ? eaf::launch_push_selftest(ws, ns, st)
+                  : eaf::launch_allreduce_selftest(ws, ns, mode, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&err_h, ws.err, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -714,6 +715,17 @@ int eaf_selftest_allreduce_timeout(int device, double timeout_ms, int mode) {
     return EAF_ECUDA;
   }
   return err_h;
+}
+
+int eaf_selftest_allreduce_timeout(int device, double timeout_ms, int mode) {
+  if (!(timeout_ms > 0.0) || timeout_ms > 10000.0 || (mode != 0 && mode != 1))
+    return EAF_EINVAL;
+  return run_wait_selftest(device, timeout_ms, mode);
+}
+
+int eaf_selftest_push_timeout(int device, double timeout_ms) {
+  if (!(timeout_ms > 0.0) || timeout_ms > 10000.0) return EAF_EINVAL;
+  return run_wait_selftest(device, timeout_ms, 2);
 }
 
 }  // extern "C"

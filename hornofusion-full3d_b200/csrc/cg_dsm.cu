@@ -438,6 +438,7 @@ struct PushSmem {
   double zero;       // z of a missing neighbour
   double dummy;      // where cells beyond the slice leave theirs
   uint64_t bar[2];
+  int gave_up;       // a block of the cluster left an exchange unfinished
 };
 static_assert(offsetof(PushSmem, rz) == 8 * kMaxClusterSize &&
                   offsetof(PushSmem, pre) == 24 * kMaxClusterSize &&
@@ -447,7 +448,7 @@ static_assert(offsetof(PushSmem, rz) == 8 * kMaxClusterSize &&
 // What a block's all-reduces need, set up once (shared-memory addresses).
 struct Pusher {
   int rank;
-  uint32_t phases;             // completion parity expected next, bit per barrier
+  uint32_t phases;             // parity of the phase that is not complete yet, bit per barrier
   uint32_t smem, bar;          // this block's PushSmem and barriers
   uint32_t to_smem, to_bar;    // those of lane's target block (lane & 15)
   uint32_t z_bytes;            // bytes of z a block receives per exchange
@@ -485,6 +486,28 @@ struct Slices {
     return 8u * (uint32_t)((cells + 1) & ~1);
   }
 };
+__device__ __forceinline__ Pusher make_pusher(const DsmArgs& a, const Slices& zs, PushSmem& ps,
+                                              int C, int rank) {
+  Pusher px;
+  const int lane = threadIdx.x & 31, to = rank - zs.reach + lane;
+  px.rank = rank;
+  px.phases = 0;
+  px.smem = smem_addr(&ps);
+  px.bar = smem_addr(&ps.bar[0]);
+  px.to_smem = cluster_map(px.smem, (uint32_t)min(lane & 15, C - 1));
+  px.to_bar = cluster_map(px.bar, (uint32_t)min(lane & 15, C - 1));
+  px.z_bytes = 0;
+  for (int b = max(0, rank - zs.reach); b <= min(C - 1, rank + zs.reach); ++b)
+    if (b != rank) px.z_bytes += zs.bytes(a, b);
+  const bool sends = lane <= 2 * zs.reach && to >= 0 && to < C && to != rank;
+  px.z_len = sends ? zs.bytes(a, rank) : 0u;
+  px.z_src = zs.slot(rank, rank);
+  px.z_dst = sends ? cluster_map(zs.slot(to, rank), (uint32_t)to) : 0u;
+  px.z_bar = sends ? cluster_map(px.bar + 8u, (uint32_t)to) : 0u;
+  px.err = a.ws.err;
+  px.timeout_ns = a.timeout_ns;
+  return px;
+}
 __device__ __forceinline__ double ld_shared_f64(uint32_t a) {
   double v;
   asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
@@ -528,6 +551,8 @@ __device__ __forceinline__ void st_shared_f64(uint32_t a, double v) {
   asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
+constexpr uint64_t kPushDrainNs = 1000000;  // bound of the wait for copies in flight
+
 // Offsets in a PushSmem, and the doubles a block's sums take there.
 constexpr uint32_t kAtPq = 0, kAtRz = 8 * kMaxClusterSize, kAtPre = 24 * kMaxClusterSize,
                    kAtWarp = 56 * kMaxClusterSize;
@@ -537,8 +562,9 @@ constexpr uint32_t kAtPq = 0, kAtRz = 8 * kMaxClusterSize, kAtPre = 24 * kMaxClu
 // waits for the partials of the (at most) CMAX blocks, whose slots beyond the
 // cluster's size hold zeros, and folds them in rank order. Two values are
 // pushed by the two halves of warp 0. The barrier's next phase, which will
-// carry `next` bytes, is opened on the way out. False if the wait gave up; a
-// block leaves as one.
+// carry `next` bytes, is opened on the way out. False if the wait gave up (the
+// phase then stays open: an arrival on it would be one too many); a block leaves
+// as one.
 template <int NV, int KIND, int CMAX>
 __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t next, Pusher& x) {
   constexpr int kPairs = (NV + 1) / 2;  // values go two by two
@@ -581,7 +607,6 @@ __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t nex
   }
   const uint32_t bar = x.bar + 8u * KIND;
   const uint32_t want = (x.phases >> KIND) & 1u;
-  x.phases ^= 1u << KIND;
   bool ok = true;
   if (!mbar_test_cluster(bar, want)) {
     const uint64_t t0 = global_ns();
@@ -598,6 +623,8 @@ __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t nex
     }
   }
   ok = __syncthreads_and(ok) != 0;
+  if (!ok) return false;
+  x.phases ^= 1u << KIND;
   if (threadIdx.x == blockDim.x - 1) push_expect(bar, next);
   const uint32_t part = x.smem + kAt;
   if (NV == 1) {
@@ -629,7 +656,30 @@ __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t nex
       v[m] = t;
     }
   }
-  return ok;
+  return true;
+}
+
+// The end of a solve, every thread of the cluster: no block leaves while another
+// may still push into its memory. After complete exchanges a barrier says so,
+// since every block has waited for all that was pushed to it. If a wait gave up,
+// pushes may be in flight behind the barrier, which all blocks' pushes precede;
+// each block then waits for the bytes that its open phases lack, with a limit far
+// beyond a copy's time because a block that gave up may never have sent them,
+// before any of them leaves.
+__device__ __forceinline__ void push_leave(PushSmem& ps, const Pusher& x, int C, bool ok) {
+  if (!ok && threadIdx.x < C) {
+    const uint32_t to = cluster_map(smem_addr(&ps.gave_up), threadIdx.x);
+    asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(to) : "memory");
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (*(volatile int*)&ps.gave_up == 0) return;
+  const uint64_t t0 = global_ns();
+  for (int b = 0; b < 2; ++b)
+    for (int n = 0; n < 4096 && !mbar_test_cluster(x.bar + 8u * b, (x.phases >> b) & 1u); ++n)
+      if (global_ns() - t0 > kPushDrainNs) break;
+  __syncthreads();
+  cluster_sync_all();
 }
 
 // Neighbour in direction d (kW..kT) of compact cell (i, j, k), or -1 at an r
@@ -693,26 +743,7 @@ __device__ void push_body(const DsmArgs& a, double* sm, PushSmem& ps, int C, int
   zs.pad = (a.chunk + 1) & ~1;
   zs.base = smem_addr(sm);
   const uint32_t own_z = zs.slot(rank, rank);
-  Pusher px;
-  {
-    const int lane = threadIdx.x & 31, to = rank - zs.reach + lane;
-    px.rank = rank;
-    px.phases = 0;
-    px.smem = smem_addr(&ps);
-    px.bar = smem_addr(&ps.bar[0]);
-    px.to_smem = cluster_map(px.smem, (uint32_t)min(lane & 15, C - 1));
-    px.to_bar = cluster_map(px.bar, (uint32_t)min(lane & 15, C - 1));
-    px.z_bytes = 0;
-    for (int b = max(0, rank - zs.reach); b <= min(C - 1, rank + zs.reach); ++b)
-      if (b != rank) px.z_bytes += zs.bytes(a, b);
-    const bool sends = lane <= 2 * zs.reach && to >= 0 && to < C && to != rank;
-    px.z_len = sends ? zs.bytes(a, rank) : 0u;
-    px.z_src = own_z;
-    px.z_dst = sends ? cluster_map(zs.slot(to, rank), (uint32_t)to) : 0u;
-    px.z_bar = sends ? cluster_map(px.bar + 8u, (uint32_t)to) : 0u;
-    px.err = err;
-    px.timeout_ns = a.timeout_ns;
-  }
+  Pusher px = make_pusher(a, zs, ps, C, rank);
   const uint32_t zero = smem_addr(&ps.zero);
   const uint32_t pq_bytes = 8u * (uint32_t)C, rz_bytes = 16u * (uint32_t)C + px.z_bytes;
   if (threadIdx.x == 0) {
@@ -895,21 +926,19 @@ __device__ void push_body(const DsmArgs& a, double* sm, PushSmem& ps, int C, int
     res->residual = residual;
     res->bnorm = bnorm;
   }
+  push_leave(ps, px, C, ok);
 }
 
 // Threads of a block whose cells (one or two each) fit its registers: one
 // cell in 96 (640 threads) or more, two in 128.
 constexpr int kPushBlock1 = 640, kPushBlock2 = 512, kPushSmall = 384;
 
-template <int R, int MAXB, int CMAX>
-__global__ void __launch_bounds__(MAXB, 1) cg_push_kernel(DsmArgs a) {
-  extern __shared__ __align__(16) double push_smem[];
-  __shared__ __align__(16) PushSmem ps;
-  const int rank = (int)cluster_ctarank(), C = (int)cluster_nctarank();
+__device__ __forceinline__ void push_init(PushSmem& ps) {
   for (int i = threadIdx.x; i < 7 * kMaxClusterSize; i += blockDim.x)
     ps.pq[i] = 0.0;  // (and rz, pre behind it)
   if (threadIdx.x == 0) {
     ps.zero = 0.0;
+    ps.gave_up = 0;
     for (int b = 0; b < 2; ++b)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&ps.bar[b]))
                    : "memory");
@@ -917,12 +946,45 @@ __global__ void __launch_bounds__(MAXB, 1) cg_push_kernel(DsmArgs a) {
   }
   // Every block's barriers exist before any block pushes.
   cluster_sync_all();
+}
+
+template <int R, int MAXB, int CMAX>
+__global__ void __launch_bounds__(MAXB, 1) cg_push_kernel(DsmArgs a) {
+  extern __shared__ __align__(16) double push_smem[];
+  __shared__ __align__(16) PushSmem ps;
+  const int rank = (int)cluster_ctarank(), C = (int)cluster_nctarank();
+  push_init(ps);
   if (*a.s.asym == 0)
     push_body<true, R, CMAX>(a, push_smem, ps, C, rank);
   else
     push_body<false, R, CMAX>(a, push_smem, ps, C, rank);
-  // No block leaves while another may still push into its memory.
-  cluster_sync_all();
+}
+
+// Self-test of an exchange that a block leaves out: two blocks of one cluster
+// complete an exchange of partials, then only block 0 enters one with z. Its wait
+// runs out, while its own partial and slice are on their way to block 1, and
+// both blocks leave through push_leave.
+constexpr int kPushTestCells = 256;  // per block
+__global__ void __launch_bounds__(64, 1) push_selftest_kernel(DsmArgs a) {
+  __shared__ __align__(16) double slices[3 * kPushTestCells];
+  __shared__ __align__(16) PushSmem ps;
+  const int rank = (int)cluster_ctarank(), C = (int)cluster_nctarank();
+  push_init(ps);
+  Slices zs;
+  zs.reach = a.reach;
+  zs.pad = a.chunk;
+  zs.base = smem_addr(slices);
+  Pusher px = make_pusher(a, zs, ps, C, rank);
+  for (int i = threadIdx.x; i < a.chunk; i += blockDim.x) slices[a.chunk + i] = 1.0;
+  const uint32_t pq_bytes = 8u * (uint32_t)C, rz_bytes = 16u * (uint32_t)C + px.z_bytes;
+  if (threadIdx.x == 0) {
+    push_expect(px.bar, pq_bytes);
+    push_expect(px.bar + 8u, rz_bytes);
+  }
+  double v[1] = {1.0}, w[2] = {1.0, 2.0};
+  bool ok = push_allsum<1, 0, 2>(v, C, pq_bytes, px) && v[0] == C * (double)blockDim.x;
+  if (ok && rank == 0) ok = push_allsum<2, 1, 2>(w, C, rz_bytes, px);
+  push_leave(ps, px, C, ok);
 }
 
 // Cells per thread of the pushed form for blocks of `block` threads, 0 where
@@ -1001,6 +1063,29 @@ bool dsm_can_launch(long long n, int block, int cluster) {
     return false;
   }
   return count >= 1;
+}
+
+cudaError_t launch_push_selftest(const GroupWs& ws, uint64_t timeout_ns, cudaStream_t st) {
+  DsmArgs a = {};
+  a.d.n = 2 * kPushTestCells;
+  a.ws = ws;
+  a.timeout_ns = timeout_ns;
+  a.chunk = kPushTestCells;
+  a.reach = 1;
+  cudaError_t e = cudaMemsetAsync(ws.err, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(64);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, push_selftest_kernel, a);
 }
 
 cudaError_t launch_cg_f64_dsm(const MeshDims& d, const SysF64& s, const GroupWs& ws,

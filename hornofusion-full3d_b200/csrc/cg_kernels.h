@@ -279,5 +279,8 @@ cudaError_t launch_barrier_selftest(const GroupWs& ws, uint64_t timeout_ns,
 // holds at least 16 doubles.
 cudaError_t launch_allreduce_selftest(const GroupWs& ws, uint64_t timeout_ns, int mode,
                                       cudaStream_t st);
+// Self-test of the cluster-resident kernel's pushed exchange (cg_dsm.cu): only
+// ws.err is used.
+cudaError_t launch_push_selftest(const GroupWs& ws, uint64_t timeout_ns, cudaStream_t st);
 
 }  // namespace eaf

@@ -551,6 +551,13 @@ int eaf_selftest_barrier_timeout(int device, double timeout_ms);
  * No reference counterpart (failure-detection test hook). */
 int eaf_selftest_allreduce_timeout(int device, double timeout_ms, int mode);
 
+/* Self-test of the cluster-resident solver's pushed exchange: of two blocks of
+ * a cluster only one enters an exchange, so its wait runs out while its own
+ * copies are in flight to the other; both must leave only after those have
+ * landed. Must return EAF_ETIMEOUT after about timeout_ms with the device
+ * context intact. No reference counterpart (failure-detection test hook). */
+int eaf_selftest_push_timeout(int device, double timeout_ms);
+
 /* Diagnostics (no reference counterpart): checks, on n generated operand
  * pairs (random over a wide exponent range, exact and near-halfway
  * quotients, zeros, infinities, NaN), that the division the TDMA sweeps use
