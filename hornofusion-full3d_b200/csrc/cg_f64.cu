@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(MAXB, 1) cg_f64_kernel(CgArgs a) {
 // The same solver with the own cells' update operands kept in shared memory
 // (cg_body's KEEP); the launcher sizes the dynamic shared memory for the
 // largest slice.
-template <int MAXB, int U, int UA>
-__global__ void __launch_bounds__(MAXB, 1) cg_keep_kernel(CgArgs a) {
+template <int MAXB, int U, int UA, int MINB = 1>
+__global__ void __launch_bounds__(MAXB, MINB) cg_keep_kernel(CgArgs a) {
   extern __shared__ __align__(16) double keep_smem[];
   Group g;
   g.counter = a.ws.counter;
@@ -1496,9 +1496,16 @@ cudaError_t launch_cg_f64_stream(const MeshDims& d, const SysF64& s, const Group
 // Where a 512-thread block's threads own at most two cells each, rounds of
 // two cells in the update phase leave no dead lanes to compute (35x70x50 on
 // 148 blocks: 6.7 against 7.0 us per iteration); every variant visits a
-// thread's cells in the same order, so all give the same bits.
+// thread's cells in the same order, so all give the same bits. Where they own
+// one, rounds of one cell fit 64 registers, and two blocks an SM: the solves
+// of two handles run side by side, which a launch on every SM would otherwise put
+// one behind the other (31,680 cells, 50 iterations, us a solve by 1, 2 and 8
+// threads: 367, 328, 316 with 128 registers, 363, 191, 169 with 64; 6.6 and 6.4
+// per iteration alone). With two cells a thread the 64 registers cost a lone
+// solve 18 % (78,540 cells: 6.9 -> 8.1).
 static const void* cg_keep_kernel_ptr(int block, long long chunk) {
   if (block <= 256) return (const void*)cg_keep_kernel<256, 4, 4>;
+  if (block <= 512 && chunk <= block) return (const void*)cg_keep_kernel<512, 1, 1, 2>;
   if (block <= 512)
     return (chunk + block - 1) / block <= 2 ? (const void*)cg_keep_kernel<512, 2, 2>
                                             : (const void*)cg_keep_kernel<512, 4, 2>;
