@@ -102,15 +102,18 @@ struct CgArgs {
 // leaves them bit-identical to sums over the live cells alone.
 
 // U: cells per thread per round of the streaming phases; UA: of the stencil
-// phase. Kernels pick them by their register budget. PF: threads 0..8 of the
+// phase. Kernels pick them by their register budget. PF: a few threads of the
 // block prefetch the block's next round of every streamed array into L2
 // (one bulk prefetch per array), for meshes whose working set exceeds L2.
-// There bytes count, and PF also moves fewer of them: phi += alpha pv of an
-// iteration is left to the next one's stencil phase, which reads that
-// direction anyway (the last one follows the loop), and the residual of the
+// There bytes count, and PF also moves fewer of them. The residual of the
 // slice's first a.keep_r cells stays in shared memory (`keep`), since only the
-// update phase uses it. 120x240x168: 128 -> 110 bytes a cell and iteration,
-// 117.9 -> 111.4 us. (L2-resident meshes lose by both: 60x120x84 11.6 -> 12.0.)
+// update phase uses it (16 bytes a kept cell). In the symmetric form (LATE),
+// phi += alpha pv of an iteration is left to the next one's stencil phase,
+// which reads that direction anyway (8 bytes a cell; the last one follows the
+// loop). 120x240x168, half of the cells kept: 128 -> 112 bytes a cell and
+// iteration, 117.9 -> 111.4 us. (L2-resident meshes lose by both: 60x120x84
+// 11.6 -> 12.0.) The seven-array form has no registers left for a late x: 134.7
+// us with it, 130.2 without, 132.5 with neither.
 // KEEP: the thread's own cells' x, r, aP and this iteration's q = A p stay
 // in the block's shared memory (`keep`, kKeepArrays x slice-length doubles)
 // for the whole solve: the stencil takes the cell's own aP from there, the
@@ -127,6 +130,7 @@ struct CgArgs {
 template <bool SYM, int U, int UA, bool PF, class G, bool KEEP = false, bool PQS = false>
 __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
   static_assert(!(PF && KEEP), "one use of the shared memory");
+  constexpr bool LATE = PF && SYM;
   const MeshDims& d = a.d;
   const SysF64& s = a.s;
   const Slice own = own_slice(d.n, g.nb, g.bid);
@@ -186,7 +190,7 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
   if (ok && !(bnorm < kSmall)) {
     double rz = v3[2];
     double beta = 0.0, alpha = 0.0;
-    bool owed = false;  // PF: phi += alpha pv of the last iteration is still to come
+    bool owed = false;  // LATE: phi += alpha pv of the last iteration is still to come
     residual = sqrt(v3[1]) / bnorm;
     if (residual != residual && a.max_iter >= 1) nan_fill = true;
     for (int iter = 1; iter <= a.max_iter && !nan_fill; ++iter) {
@@ -233,17 +237,17 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
         owed = false;
         auto pnew = [z, pold, bt](int cc) { return z[cc] + bt * pold[cc]; };
         for (int c0 = own.begin + (int)threadIdx.x; c0 < own.end; c0 += B * UA) {
-          if (PF && threadIdx.x < 9) {
+          if (PF && threadIdx.x < (LATE ? 9 : 8)) {
             const int nl = c0 - (int)threadIdx.x + B * UA, nh = min(nl + B * UA, own.end);
-            const double* arr[9] = {z, pold, aP, A.aE, A.aN, A.aT, x, z, pold};
-            const int off = threadIdx.x >= 7 ? d.plane : 0;
+            const double* arr[9] = {z, pold, aP, A.aE, A.aN, A.aT, z, pold, x};
+            const int off = threadIdx.x == 6 || threadIdx.x == 7 ? d.plane : 0;
             l2_prefetch_cells(arr[threadIdx.x], nl + off, nh + off, d.n);
           }
           double qv[UA], pc[UA], xn[UA];
 #pragma unroll
           for (int u = 0; u < UA; ++u) {
             const int c = min(c0 + u * B, last);
-            if (PF) {
+            if (LATE) {
               const double po = pold[c];
               pc[u] = z[c] + bt * po;
               xn[u] = x[c] + al * po;
@@ -263,7 +267,7 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
               } else {
                 q[c0 + u * B] = qv[u];
               }
-              if (PF) x[c0 + u * B] = xn[u];
+              if (LATE) x[c0 + u * B] = xn[u];
             }
             v1[0] = v1[0] + (live ? pc[u] * qv[u] : 0.0);
           }
@@ -280,14 +284,14 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
       const double pq = v1[0];
       if (fabs(pq) < kSmall) break;
       alpha = rz / pq;
-      owed = PF;
+      owed = LATE;
       // Phase B: phi += alpha pv; r -= alpha q; r.r; z and r.z (:538-553)
       double v2[2] = {0.0, 0.0};
       for (int c0 = own.begin + (int)threadIdx.x; c0 < own.end; c0 += B * U) {
-        if (PF && threadIdx.x < 3) {
+        if (PF && threadIdx.x < (LATE ? 3 : 5)) {
           const int nl = c0 - (int)threadIdx.x + B * U, nh = min(nl + B * U, own.end);
-          const double* arr[3] = {q, aP, r};
-          if (threadIdx.x < 2 || nl - own.begin >= a.keep_r)
+          const double* arr[5] = {q, aP, r, pcur, x};
+          if (threadIdx.x != 2 || nl - own.begin >= a.keep_r)
             l2_prefetch_cells(arr[threadIdx.x], nl, nh, d.n);
         }
         double pv[U], qv[U], dv[U], xv[U], rv[U];
@@ -305,10 +309,10 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
             xv[u] = kx[o];
             rv[u] = kr[o];
           } else {
-            pv[u] = PF ? 0.0 : pcur[c];
+            pv[u] = LATE ? 0.0 : pcur[c];
             qv[u] = q[c];
             dv[u] = aP[c];
-            xv[u] = PF ? 0.0 : x[c];
+            xv[u] = LATE ? 0.0 : x[c];
             rv[u] = rr[c];
           }
         }
@@ -324,7 +328,7 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
               kx[c - own.begin] = xn;
               kr[c - own.begin] = rn;
             } else {
-              if (!PF) x[c] = xn;
+              if (!LATE) x[c] = xn;
               rr[c] = rn;
             }
             z[c] = zv;
@@ -344,7 +348,7 @@ __device__ void cg_body(const CgArgs& a, G& g, double* keep = nullptr) {
       beta = v2[1] / guard_small(rz);
       rz = v2[1];
     }
-    if (PF && owed && !nan_fill) {  // the last iteration's phi += alpha pv
+    if (LATE && owed && !nan_fill) {  // the last iteration's phi += alpha pv
       const double* __restrict__ p = (n_iter & 1) ? s.p : s.p2;
       for (int c = own.begin + (int)threadIdx.x; c < own.end; c += B) x[c] = x[c] + alpha * p[c];
     }
