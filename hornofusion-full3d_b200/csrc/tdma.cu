@@ -181,6 +181,11 @@ struct SweepArgs {
 constexpr int kEmptyHigh = 0x7ff00001;
 __device__ __forceinline__ double empty_slot() { return __hiloint2double(kEmptyHigh, kEmptyHigh); }
 __device__ __forceinline__ bool is_empty(double v) { return __double2hiint(v) == kEmptyHigh; }
+// A caller's value as a slot may carry it: one with the mark's bits becomes the
+// quiet NaN that any operation on it makes of it.
+__device__ __forceinline__ double unmarked(double v) {
+  return is_empty(v) ? __hiloint2double(kEmptyHigh | 0x00080000, __double2loint(v)) : v;
+}
 __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
@@ -647,6 +652,9 @@ __device__ void fetch_mail(const SweepArgs& a, double* ring, int lane) {
       Patience wait;
       while (!__all_sync(kAllLanes, slot_free<K>(to)))
         if (wait.gives_up(a.err, a.timeout_ns)) return;
+      // (looked at here, not as they are loaded: a look waits for its load)
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = unmarked(v[k]);
       st_pairs(to, v);
     }
   }
