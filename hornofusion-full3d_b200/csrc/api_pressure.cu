@@ -161,7 +161,7 @@ int run_assemble(eaf_cg* h, const eaf_assembly_fields_t& f) {
                         sizeof(double) * eaf::assembly_scratch_doubles(h->nr, h->nth, h->nz)));
   }
   EAF_CUDA(cudaEventRecord(h->ev[2], h->st));
-  EAF_CUDA(eaf::launch_assemble_f64(f, h->nr, h->nth, h->nz, h->asm_s,
+  EAF_CUDA(eaf::launch_assemble_f64(f, h->nr, h->nth, h->nz, h->stage, h->asm_s,
                                     &h->ws.result[1].residual, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   h->last_kernels = 4;
@@ -279,7 +279,7 @@ int run_step(eaf_cg* h, const eaf_assembly_fields_t& d, double alpha_p, int max_
   for (int i = 0; i < 2; ++i)
     if (!h->step_ev[i]) EAF_CUDA(cudaEventCreate(&h->step_ev[i]));
   EAF_CUDA(cudaEventRecord(h->step_ev[0], h->st));
-  EAF_CUDA(eaf::launch_assemble_f64(d, h->nr, h->nth, h->nz, h->asm_s,
+  EAF_CUDA(eaf::launch_assemble_f64(d, h->nr, h->nth, h->nz, h->stage, h->asm_s,
                                     &h->ws.result[1].residual, h->st));
   HaloInputs in = {d.aW, d.aE, d.aS, d.aN, d.aB, d.aT, d.aP, d.Su, d.pp};
   SolveOpts o = {false, max_iter, 0, tol, 0.0};

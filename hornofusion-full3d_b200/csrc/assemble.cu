@@ -528,15 +528,17 @@ unsigned asm_grid(long long work) {
 
 }  // namespace
 
-// Scratch: 4 gradient arrays, 12 face arrays (6 per phase), 6 of quotients, the
-// open bits and the block partials.
+// Scratch: one gradient array, 12 face arrays (6 per phase), the open bits and the
+// block partials. The other three gradients and the six arrays of quotients go
+// to the caller's nine.
 size_t assembly_scratch_doubles(int nr, int nth, int nz) {
   const size_t nh = (size_t)(nr + 4) * (nth + 4) * (nz + 4);
-  return 22 * nh + (nh + 7) / 8 + 2 * 148 * 8;
+  return 13 * nh + (nh + 7) / 8 + 2 * 148 * 8;
 }
 
 cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth, int nz,
-                                double* scratch, double* result, cudaStream_t st) {
+                                double* const* halo9, double* scratch, double* result,
+                                cudaStream_t st) {
   AsmArgs a;
   a.f = f;
   a.nr = nr;
@@ -548,9 +550,9 @@ cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth,
   a.nh = a.sxy * (unsigned)(nz + 4);
   double* w = scratch;
   auto take = [&](size_t n) { double* r = w; w += n; return r; };
-  a.gr = take(a.nh);
-  a.gth = take(a.nh);
-  a.gz_l = take(a.nh);
+  a.gr = halo9[0];
+  a.gth = halo9[1];
+  a.gz_l = halo9[2];
   a.gz_g = take(a.nh);
   for (FacePhase* F : {&a.fl, &a.fg}) {
     F->cW = take(a.nh);
@@ -561,8 +563,8 @@ cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth,
     F->fB = take(a.nh);
   }
   for (int m = 0; m < 3; ++m) {
-    a.dl[m] = take(a.nh);
-    a.dg[m] = take(a.nh);
+    a.dl[m] = halo9[3 + m];
+    a.dg[m] = halo9[6 + m];
   }
   a.open = reinterpret_cast<unsigned char*>(take((a.nh + 7) / 8));
   a.fd_sx = FastDiv(a.sx);

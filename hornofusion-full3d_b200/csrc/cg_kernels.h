@@ -260,13 +260,15 @@ cudaError_t run_div_check(long long n, unsigned long long seed, unsigned long lo
 cudaError_t launch_pcorr_f64(const eaf_pcorr_fields_t& f, int nr, int nth, int nz,
                              cudaStream_t st);
 
-// Pressure-equation assembly (solve_pressure_correction before the CG), three
-// launches on `st` into device pointers of `f`; `scratch` holds
-// assembly_scratch_doubles() doubles (gradients, quotients, faces, block partials), the
+// Pressure-equation assembly (solve_pressure_correction before the CG), four
+// launches on `st` into device pointers of `f`; `halo9` are nine halo-layout
+// arrays that are overwritten (gradients, quotients), `scratch` holds
+// assembly_scratch_doubles() doubles (a gradient, faces, block partials), the
 // residual goes to `result` (the device address of pinned memory, or device memory).
 size_t assembly_scratch_doubles(int nr, int nth, int nz);
 cudaError_t launch_assemble_f64(const eaf_assembly_fields_t& f, int nr, int nth, int nz,
-                                double* scratch, double* result, cudaStream_t st);
+                                double* const* halo9, double* scratch, double* result,
+                                cudaStream_t st);
 
 // Threads per block of the batched kernels (FP64 and mixed).
 constexpr int kBatchBlock = 512;

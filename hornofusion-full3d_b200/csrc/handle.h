@@ -15,7 +15,8 @@ struct eaf_cg {
   eaf::MeshDims d;
   size_t nh;  // halo-layout elements per array
   cudaStream_t st;
-  double* stage[9];  // aW aE aS aN aB aT aP Su phi, halo layout (host path)
+  double* stage[9];  // aW aE aS aN aB aT aP Su phi, halo layout (host path); the
+                     // assembly's gradients and quotients, whose inputs are elsewhere
   eaf::SysF64 s;
   eaf::SysF32 f;
   bool have_f32;
@@ -41,7 +42,7 @@ struct eaf_cg {
   int form;          // EAF_CG_FORM_*: the FP64 solver's recurrences
   double* asm_d;     // assembly mirror: doubles (lazy)
   int* asm_i;        // assembly mirror: ints (lazy)
-  double* asm_s;     // assembly scratch: gradients, partials, residual (lazy)
+  double* asm_s;     // assembly scratch: a gradient, faces, partials (lazy)
   cudaEvent_t step_ev[2];  // span of a whole pressure step (lazy)
 };
 
