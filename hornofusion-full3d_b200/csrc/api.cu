@@ -61,10 +61,7 @@ using eaf::set_error;
 
 static void free_handle(eaf_cg* h) {
   for (int i = 0; i < 9; ++i) cudaFree(h->stage[i]);
-  double* f64[] = {h->s.aP, h->s.aE, h->s.aN, h->s.aT, h->s.aW, h->s.aS, h->s.aB,
-                   h->s.b,  h->s.x,  h->s.r,  h->s.p,  h->s.q,  h->s.p2, h->s.z,
-                   h->s.s0, h->s.s1, h->s.dinv};
-  for (double* p : f64) cudaFree(p);
+  cudaFree(h->sys);
   cudaFree(h->s.asym);
   float* f32[] = {h->f.aP, h->f.aE, h->f.aN, h->f.aT, h->f.aW, h->f.aS, h->f.aB,
                   h->f.r,  h->f.z,  h->f.q,  h->f.e,  h->f.p,  h->f.p2};
@@ -72,7 +69,7 @@ static void free_handle(eaf_cg* h) {
   cudaFree(h->ws.part);
   cudaFree(h->ws.counter);
   cudaFree(h->ws.err);
-  cudaFree(h->tdma_mbox);
+  cudaFree(h->tdma_more);
   cudaFree(h->pc_d);
   cudaFree(h->pc_i);
   cudaFree(h->asm_d);
@@ -316,7 +313,16 @@ int eaf_cg_create_mesh(eaf_cg_t* out, int nr, int nth, int nz, int is_parallel,
                     &h->s.dinv};
   // One padding cell (two, rounded) past each compact array: the streaming
   // kernel's bulk copies move whole 16-byte pairs of cells.
-  for (double** p : f64) alloc((void**)p, (size_t)(n + 2) * sizeof(double));
+  const size_t stride = ((size_t)n + 2 + 31) / 32 * 32;
+  h->sys_doubles = stride * (sizeof(f64) / sizeof(f64[0]));
+  alloc((void**)&h->sys, h->sys_doubles * sizeof(double));
+  if (e == cudaSuccess) {
+    double* at = h->sys;
+    for (double** p : f64) {
+      *p = at;
+      at += stride;
+    }
+  }
   alloc((void**)&h->s.asym, sizeof(int));
   int dev_sms = 0;
   if (e == cudaSuccess)

@@ -20,26 +20,70 @@ namespace {
 // ---------------------------------------------------------------------------
 // Line-by-line TDMA sweeps and the transport residual on the handle's mesh.
 // ---------------------------------------------------------------------------
-int enqueue_tdma(eaf_cg* h, const HaloInputs& in, double* phi, int n_sweep) {
-  if (!h->tdma_mbox) {  // the mailboxes and the records, in one allocation
-    const size_t mbox =
-        (eaf::tdma_mailbox_doubles(h->nr, h->nth, h->nz) + 31) / 32 * 32;
-    EAF_CUDA(cudaMalloc((void**)&h->tdma_mbox,
-                        sizeof(double) *
-                            (mbox + eaf::tdma_factor_doubles(h->nr, h->nth, h->nz))));
-    h->tdma_fac = h->tdma_mbox + mbox;
+cudaError_t grow_tdma(eaf_cg* h, size_t doubles) {
+  if (h->tdma_more_doubles >= doubles) return cudaSuccess;
+  double* p = nullptr;
+  const cudaError_t e = cudaMalloc((void**)&p, doubles * sizeof(double));
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return e;
   }
+  cudaFree(h->tdma_more);
+  h->tdma_more = p;
+  h->tdma_more_doubles = doubles;
+  return cudaSuccess;
+}
+
+// Scratch of a call. The hand-over slots, the old values and the records of one
+// direction (about 14 doubles a cell) lie in the solver's compact arrays (17),
+// which hold nothing between solves, or, on meshes too thin for that, beside
+// them. A call of one sweep uses every record once and needs no more. One of
+// several keeps the other two directions' records too (about 19 doubles a cell,
+// allocated by the first such call), or, where they find no room, builds each
+// direction's again before its sweep.
+cudaError_t tdma_scratch(eaf_cg* h, int n_sweep, eaf::TdmaScratch* w) {
+  const eaf::TdmaSizes z = eaf::tdma_sizes(h->nr, h->nth, h->nz);
+  int big = 0;
+  for (int d = 1; d < 3; ++d)
+    if (z.rec[d] > z.rec[big]) big = d;
+  const size_t one = z.mail + z.old + z.rec[big];
+  const bool in_sys = one <= h->sys_doubles;
+  const size_t least = in_sys ? 0 : one;
+  w->rebuild = n_sweep < 2;
+  cudaError_t e = cudaSuccess;
+  if (!w->rebuild) {
+    e = grow_tdma(h, least + z.rec[0] + z.rec[1] + z.rec[2] - z.rec[big]);
+    w->rebuild = e == cudaErrorMemoryAllocation;
+  }
+  if (w->rebuild) e = grow_tdma(h, least);
+  if (e != cudaSuccess) return e;
+  double* at = in_sys ? h->sys : h->tdma_more;
+  w->mail = at;
+  w->old = at + z.mail;
+  w->rec[0] = w->rec[1] = w->rec[2] = at + z.mail + z.old;
+  double* more = h->tdma_more + least;
+  for (int d = 0; d < 3 && !w->rebuild; ++d) {
+    if (d == big) continue;
+    w->rec[d] = more;
+    more += z.rec[d];
+  }
+  return cudaSuccess;
+}
+
+int enqueue_tdma(eaf_cg* h, const HaloInputs& in, double* phi, int n_sweep) {
+  eaf::TdmaScratch w;
+  EAF_CUDA(tdma_scratch(h, n_sweep, &w));
   eaf::tdma_launch_shape(h->nr, h->nth, h->nz, h->sms, &h->last_grid, &h->last_block);
   h->last_cluster = 1;
   EAF_CUDA(cudaEventRecord(h->ev[1], h->st));
   EAF_CUDA(cudaEventRecord(h->ev[2], h->st));
   if (n_sweep > 0) {
-    EAF_CUDA(eaf::launch_tdma_f64(in, phi, h->nr, h->nth, h->nz, n_sweep, h->tdma_mbox,
-                                  h->tdma_fac, h->sms, h->ws, h->timeout_ns, h->st));
+    EAF_CUDA(eaf::launch_tdma_f64(in, phi, h->nr, h->nth, h->nz, n_sweep, w, h->sms, h->ws,
+                                  h->timeout_ns, h->st));
   }
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(cudaEventRecord(h->ev[4], h->st));
-  h->last_kernels = n_sweep > 0 ? 3 + 6 * n_sweep : 0;
+  h->last_kernels = n_sweep > 0 ? (w.rebuild ? 9 : 6) * n_sweep + (w.rebuild ? 0 : 3) : 0;
   return EAF_OK;
 }
 

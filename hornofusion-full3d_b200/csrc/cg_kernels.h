@@ -233,16 +233,22 @@ cudaError_t launch_batch_mixed(const BatchTables& t, int grid, int block,
                                double inner_tol, uint64_t timeout_ns, cudaStream_t st);
 const void* batch_f64_kernel_ptr();
 // Line-by-line TDMA sweeps (tdma_3d_mpi, serial) on halo-layout arrays, in
-// place on phi: three launches of line records (`fac`, tdma_factor_doubles()
-// doubles, computed from the coefficients), then one cooperative launch per
-// direction and sweep. `mbox` holds tdma_mailbox_doubles() doubles of line
-// hand-over slots. Every mesh extent at most 1024. tdma_launch_shape: the
-// largest grid and block of the sweep launches.
-size_t tdma_mailbox_doubles(int nr, int nth, int nz);
-size_t tdma_factor_doubles(int nr, int nth, int nz);
+// place on phi: three launches of line records, computed from the
+// coefficients, then per direction and sweep one of old values and a cooperative
+// one. `rebuild`: the three directions' records share their memory, and each is
+// built before its direction in every sweep. Every mesh extent at most 1024.
+// tdma_launch_shape: the largest grid and block of the sweep launches.
+struct TdmaSizes {
+  size_t mail, old, rec[3];  // doubles, multiples of 32
+};
+struct TdmaScratch {
+  double *mail, *old, *rec[3];  // line hand-over slots, a direction's old values, records
+  bool rebuild;
+};
+TdmaSizes tdma_sizes(int nr, int nth, int nz);
 void tdma_launch_shape(int nr, int nth, int nz, int sms, int* grid, int* block);
 cudaError_t launch_tdma_f64(const HaloInputs& in, double* phi, int nr, int nth, int nz,
-                            int n_sweep, double* mbox, double* fac, int sms, const GroupWs& ws,
+                            int n_sweep, const TdmaScratch& w, int sms, const GroupWs& ws,
                             uint64_t timeout_ns, cudaStream_t st);
 // compute_residual_3d_mpi (serial) into ws.result->residual, on the grid that
 // residual_launch_shape gives for n cells.

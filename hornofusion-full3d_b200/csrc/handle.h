@@ -17,6 +17,8 @@ struct eaf_cg {
   cudaStream_t st;
   double* stage[9];  // aW aE aS aN aB aT aP Su phi, halo layout (host path); the
                      // assembly's gradients and quotients, whose inputs are elsewhere
+  double* sys;         // the arrays of s, one behind the other; between solves,
+  size_t sys_doubles;  // scratch of the TDMA sweeps
   eaf::SysF64 s;
   eaf::SysF32 f;
   bool have_f32;
@@ -35,8 +37,8 @@ struct eaf_cg {
   double last_solve_ms, last_kernel_ms, last_e2e_ms;
   int last_sym, last_kernels;
   int last_grid, last_block, last_cluster;
-  double* tdma_mbox;  // TDMA line hand-over slots (lazy)
-  double* tdma_fac;   // TDMA line records, behind them
+  double* tdma_more;  // TDMA scratch beyond `sys` (lazy)
+  size_t tdma_more_doubles;
   double* pc_d;      // post-CG correction mirror: doubles (lazy)
   int* pc_i;         // post-CG correction mirror: ints (lazy)
   int form;          // EAF_CG_FORM_*: the FP64 solver's recurrences

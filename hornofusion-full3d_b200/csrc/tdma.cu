@@ -44,7 +44,8 @@
 // Layout. The sweep itself is bound by latency, so the transposing work is
 // left to parallel kernels before it: what does not depend on phi -- the
 // guarded pivots m_i, cp_i, y_i = 1/m_i (by the same fixed-point passes) and
-// the scan's segment products -- is computed once per call into a record per
+// the scan's segment products -- is computed once per call (before a direction's
+// sweep where the records of only one have room) into a record per
 // line and direction, lane by lane; what a direction takes from the old phi
 // (its plus-side neighbours, which no line changes before it is solved) goes
 // into an old-value record per line before each direction. A line is then two
@@ -1184,23 +1185,16 @@ cudaError_t launch_sweep(SweepArgs a, int sms, cudaStream_t st) {
 
 }  // namespace
 
-size_t tdma_mailbox_doubles(int nr, int nth, int nz) {
-  size_t most = 0;
-  for (int dir = 0; dir < 3; ++dir) {
-    const size_t n = dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir)).mail;
-    if (n > most) most = n;
-  }
-  return most;
-}
-
-size_t tdma_factor_doubles(int nr, int nth, int nz) {
-  size_t sum = 0, old = 0;
+TdmaSizes tdma_sizes(int nr, int nth, int nz) {
+  TdmaSizes z = {};
+  auto rounded = [](size_t n) { return (n + 31) / 32 * 32; };
   for (int dir = 0; dir < 3; ++dir) {
     const DirSizes s = dir_sizes(make_dir(HaloInputs{}, nr, nth, nz, dir));
-    sum += s.rec;
-    if (s.old > old) old = s.old;
+    z.rec[dir] = rounded(s.rec);
+    if (s.mail > z.mail) z.mail = rounded(s.mail);
+    if (s.old > z.old) z.old = rounded(s.old);
   }
-  return sum + old;  // every direction's records, one direction's old values
+  return z;
 }
 
 void tdma_launch_shape(int nr, int nth, int nz, int sms, int* grid, int* block) {
@@ -1215,45 +1209,50 @@ void tdma_launch_shape(int nr, int nth, int nz, int sms, int* grid, int* block) 
 }
 
 cudaError_t launch_tdma_f64(const HaloInputs& in, double* phi, int nr, int nth, int nz,
-                            int n_sweep, double* mbox, double* fac, int sms, const GroupWs& ws,
+                            int n_sweep, const TdmaScratch& w, int sms, const GroupWs& ws,
                             uint64_t timeout_ns, cudaStream_t st) {
   if (nr > kTdmaMaxLine || nth > kTdmaMaxLine || nz > kTdmaMaxLine)
     return cudaErrorInvalidValue;
   std::lock_guard<std::mutex> attr_lock(launch_attr_mutex());
   (void)cudaGetLastError();  // report these launches' errors, not an older one
-  const double* rec[3];
-  for (int dir = 0; dir < 3; ++dir) {
+  // A direction's records; the call's first launch also refreshes phi's theta
+  // halos and clears the error word.
+  auto build = [&](int dir, bool first) {
     FactorArgs f;
     f.d = make_dir(in, nr, nth, nz, dir);
-    f.rec = fac;
-    f.mail = mbox;
-    f.phi = dir == 0 ? phi : nullptr;
-    f.err = dir == 0 ? ws.err : nullptr;
+    f.rec = w.rec[dir];
+    f.mail = w.mail;
+    f.phi = first ? phi : nullptr;
+    f.err = first ? ws.err : nullptr;
     f.nr = nr;
     f.nth = nth;
     f.nz = nz;
-    rec[dir] = fac;
-    fac += dir_sizes(f.d).rec;
-    const cudaError_t e = with_k(f.d.L, [&](auto k) {
+    return with_k(f.d.L, [&](auto k) {
       constexpr int K = decltype(k)::value;
       f.g = line_geo<K>(f.d.L);
       return launch_tiles(tdma_factor_kernel<K>, f, f.g.rec, st);
     });
+  };
+  for (int dir = 0; dir < 3 && !w.rebuild; ++dir) {
+    const cudaError_t e = build(dir, dir == 0);
     if (e != cudaSuccess) return e;
   }
-  double* const old = fac;
   for (int sweep = 1; sweep <= n_sweep; ++sweep) {
     for (int dir = 0; dir < 3; ++dir) {
+      if (w.rebuild) {
+        const cudaError_t e = build(dir, sweep == 1 && dir == 0);
+        if (e != cudaSuccess) return e;
+      }
       OldArgs o;
       o.d = make_dir(in, nr, nth, nz, dir);
       o.phi = phi;
-      o.old = old;
+      o.old = w.old;
       SweepArgs a;
       a.d = o.d;
       if (dir == 2 && sweep == n_sweep) a.d.wrap = 0;  // no refresh after the last direction
-      a.rec = rec[dir];
-      a.old = old;
-      a.mail = mbox;
+      a.rec = w.rec[dir];
+      a.old = w.old;
+      a.mail = w.mail;
       a.phi = phi;
       a.err = ws.err;
       a.timeout_ns = timeout_ns;
