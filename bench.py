@@ -376,10 +376,8 @@ def run_ours(args, rank, world, local_rank):
         "e2e": {"value": e2e_ci / (e2e_ms / 1e3), "unit": "cell-iters/s",
                 "h2d_bytes_per_step": 9 * halo_bytes,
                 "d2h_bytes_per_step": halo_bytes + 40},
-        # pack, solver, unpack; the flat kernels' launcher also fills the
-        # p.q slot sets with the empty-slot marker (one small kernel)
-        "gpu_launches": (4 if kernel in ("cg_keep_kernel", "cg_f64_kernel")
-                         and 1 < plan[0] <= 160 else 3) * args.steps,
+        # pack, solver (with the kernel that clears its slots), unpack
+        "gpu_launches": solver.last_timing()["kernels"] * args.steps,
         "clocks": clk,
     }
     print(json.dumps(line), flush=True)
@@ -493,6 +491,7 @@ def run_tdma(args):
             t = cg.last_timing()
             ms += t["solve_ms"]
             kms += t["kernel_ms"]
+        kernels = t["kernels"]
         e2e = 0.0
         for _ in range(args.steps):
             host[8][...] = 0.0
@@ -526,8 +525,8 @@ def run_tdma(args):
         "elements_per_sweep": crit,
         "ns_per_element": 1e6 * (kms / args.steps) / ns / crit,
         "note": "lines of one direction run as a wavefront: (A+B-1) dependent line "
-                "solves of L elements each, one sequential Thomas step per element"}
-    line["gpu_launches"] = 2 * args.steps
+                "solves of L elements each, a warp a line"}
+    line["gpu_launches"] = kernels * args.steps
     print(json.dumps(line), flush=True)
     return 0
 
@@ -753,6 +752,7 @@ def run_pstep(args):
             kms += cg.last_timing()["kernel_ms"]
             iters.append(nit)
         cg_kernel = solver_kernel_name(cg, cg.last_launch())
+        kernels = cg.last_timing()["kernels"]
         e2e = 0.0
         h = _pinned_fields(eaf, f0)
         for _ in range(args.steps):
@@ -798,9 +798,7 @@ def run_pstep(args):
                             "kind": "port",
                             "sample": f"oracle port: assembly and corrections on one thread, "
                                       f"CG on {cores} threads, one step, {cpu_s:.2f} s"}
-    # assembly 4; pack, solver, unpack (+ the p.q slot fill of a flat grid); corrections 3
-    cg_launches = 4 if cg_kernel in ("cg_keep_kernel", "cg_f64_kernel") else 3
-    line["gpu_launches"] = (4 + cg_launches + 3) * args.steps
+    line["gpu_launches"] = kernels * args.steps  # assembly, CG, corrections
     print(json.dumps(line), flush=True)
     return 0
 

@@ -225,8 +225,12 @@ bool runs_resident(const SolverLaunch& L, long long n, bool allowed) {
 
 cudaError_t launch_f64_solver(const SolverLaunch& L, int resident, const MeshDims& d,
                               const SysF64& s, const GroupWs& ws, size_t slot_doubles,
-                              int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st) {
-  if (runs_resident(L, d.n, resident != 0))
+                              int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st,
+                              int* kernels) {
+  const bool in_cluster = runs_resident(L, d.n, resident != 0);
+  // (the others clear their counter, slots and error word by a kernel)
+  if (kernels) *kernels = in_cluster || (L.cluster <= 1 && !L.slots && L.stream) ? 1 : 2;
+  if (in_cluster)
     return launch_cg_f64_dsm(d, s, ws, max_iter, tol, L.block, L.cluster, st,
                              resident == 2 ? kDsmSignalMbarrier : kDsmSignalDefault,
                              timeout_ns);
@@ -533,7 +537,7 @@ static int ensure_f32(eaf_cg* h) {
 int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts& o) {
   EAF_CUDA(cudaEventRecord(h->ev[1], h->st));
   EAF_CUDA(eaf::launch_pack_f64(h->d, in, h->s, h->st));
-  int grid, block, cluster = 1;
+  int grid, block, cluster = 1, kernels = 1;
   if (o.mixed) {
     int rc = ensure_f32(h);
     if (rc != EAF_OK) return rc;
@@ -559,7 +563,7 @@ int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts&
     else
       EAF_CUDA(eaf::launch_f64_solver(L, h->resident, h->d, h->s, h->ws,
                                       kPartTableDoubles(h), o.max_iter, o.tol,
-                                      h->timeout_ns, h->st));
+                                      h->timeout_ns, h->st, &kernels));
   }
   h->last_grid = grid;
   h->last_block = block;
@@ -567,7 +571,7 @@ int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts&
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(eaf::launch_unpack_f64(h->d, h->s.x, phi, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[4], h->st));
-  h->last_kernels = 3;
+  h->last_kernels = 2 + kernels;  // pack, the solver's, unpack
   return EAF_OK;
 }
 

@@ -114,7 +114,7 @@ int run_residual(eaf_cg* h, const HaloInputs& in, const double* phi, double* res
   EAF_CUDA(cudaStreamSynchronize(h->st));
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, h->ev[2], h->ev[3]) == cudaSuccess) h->last_kernel_ms = ms;
-  h->last_kernels = 1;
+  h->last_kernels = 2;  // the group's words, the residual
   *residual = h->res_h->residual;
   return h->res_h->status;
 }

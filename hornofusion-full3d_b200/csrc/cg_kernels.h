@@ -175,10 +175,11 @@ bool runs_resident(const SolverLaunch& L, long long n, bool allowed);
 // Enqueues the plain FP64 solver (reference form) on launch L: the flat,
 // cluster or cluster-resident kernel; `slot_doubles` is the size of ws.part.
 // `resident`: 0 never the cluster-resident kernel, 1 it with its default
-// signalling, 2 it with mbarrier signalling.
+// signalling, 2 it with mbarrier signalling. `kernels`: how many were launched.
 cudaError_t launch_f64_solver(const SolverLaunch& L, int resident, const MeshDims& d,
                               const SysF64& s, const GroupWs& ws, size_t slot_doubles,
-                              int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st);
+                              int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st,
+                              int* kernels = nullptr);
 // Single-reduction (Chronopoulos-Gear) form of the same PCG: one group
 // all-reduce per iteration; uses s0/s1 and reuses r, z, q, p2 as the
 // double-buffered r and w = A M^-1 r.
