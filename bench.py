@@ -83,7 +83,8 @@ def measured_peaks():
 def solver_kernel_name(solver, plan):
     """Name of the persistent kernel the last solve of `solver` ran."""
     if len(plan) > 2:
-        return "cg_push_kernel or cg_dsm_kernel" if plan[0] == plan[2] else "cg_cluster_kernel"
+        return {solver.RAN_NOT_RESIDENT: "cg_cluster_kernel",
+                solver.RAN_PUSHED: "cg_push_kernel"}.get(solver.last_resident(), "cg_dsm_kernel")
     return {solver.KERNEL_LOADS: "cg_f64_kernel", solver.KERNEL_STREAM: "cg_stream_kernel",
             solver.KERNEL_SLOTS: "cg_cluster_kernel",
             solver.KERNEL_KEEP: "cg_keep_kernel"}[solver.last_kernel()]

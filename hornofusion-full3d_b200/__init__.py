@@ -270,6 +270,17 @@ class CGSolver:
         (RESIDENT_OFF); all give the same bits."""
         check(self._lib.eaf_cg_set_resident(self._h, int(mode)), "set_resident")
 
+    RAN_NOT_RESIDENT = 0
+    RAN_CLUSTER_BARRIER = 1
+    RAN_MBARRIER = 2
+    RAN_PUSHED = 3
+
+    def last_resident(self) -> int:
+        """Form of the cluster-resident kernel that the last solve ran (RAN_*)."""
+        k = ctypes.c_int()
+        check(self._lib.eaf_cg_last_resident(self._h, ctypes.byref(k)), "last_resident")
+        return k.value
+
     def mixed_trace(self, max_steps: int = 1000) -> list:
         """Per refinement step of the last mixed-precision solve: inner FP32
         iterations, the inner CG's residual reduction and the FP64 outer

@@ -226,14 +226,17 @@ bool runs_resident(const SolverLaunch& L, long long n, bool allowed) {
 cudaError_t launch_f64_solver(const SolverLaunch& L, int resident, const MeshDims& d,
                               const SysF64& s, const GroupWs& ws, size_t slot_doubles,
                               int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st,
-                              int* kernels) {
+                              SolverRan* ran) {
   const bool in_cluster = runs_resident(L, d.n, resident != 0);
-  // (the others clear their counter, slots and error word by a kernel)
-  if (kernels) *kernels = in_cluster || (L.cluster <= 1 && !L.slots && L.stream) ? 1 : 2;
+  if (ran) {
+    // (the others clear their counter, slots and error word by a kernel)
+    ran->kernels = in_cluster || (L.cluster <= 1 && !L.slots && L.stream) ? 1 : 2;
+    ran->resident = EAF_CG_RESIDENT_NONE;
+  }
   if (in_cluster)
     return launch_cg_f64_dsm(d, s, ws, max_iter, tol, L.block, L.cluster, st,
                              resident == 2 ? kDsmSignalMbarrier : kDsmSignalDefault,
-                             timeout_ns);
+                             timeout_ns, ran ? &ran->resident : nullptr);
   if (L.cluster > 1 || L.slots)
     return launch_cg_f64_cluster(d, s, ws, ws.part, slot_doubles, max_iter, tol, timeout_ns,
                                  L.grid, L.block, L.cluster, st);
@@ -440,6 +443,12 @@ int eaf_cg_set_resident(eaf_cg_t h, int resident) {
   return EAF_OK;
 }
 
+int eaf_cg_last_resident(eaf_cg_t h, int* form) {
+  if (!h || !form) return EAF_EINVAL;
+  *form = h->last_resident;
+  return EAF_OK;
+}
+
 int eaf_cg_last_cluster(eaf_cg_t h, int* cluster_blocks) {
   if (!h || !cluster_blocks) return EAF_EINVAL;
   *cluster_blocks = h->last_cluster > 0 ? h->last_cluster : 1;
@@ -537,7 +546,8 @@ static int ensure_f32(eaf_cg* h) {
 int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts& o) {
   EAF_CUDA(cudaEventRecord(h->ev[1], h->st));
   EAF_CUDA(eaf::launch_pack_f64(h->d, in, h->s, h->st));
-  int grid, block, cluster = 1, kernels = 1;
+  int grid, block, cluster = 1;
+  eaf::SolverRan ran = {1, EAF_CG_RESIDENT_NONE};
   if (o.mixed) {
     int rc = ensure_f32(h);
     if (rc != EAF_OK) return rc;
@@ -563,7 +573,7 @@ int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts&
     else
       EAF_CUDA(eaf::launch_f64_solver(L, h->resident, h->d, h->s, h->ws,
                                       kPartTableDoubles(h), o.max_iter, o.tol,
-                                      h->timeout_ns, h->st, &kernels));
+                                      h->timeout_ns, h->st, &ran));
   }
   h->last_grid = grid;
   h->last_block = block;
@@ -571,7 +581,8 @@ int enqueue_solve(eaf_cg* h, const HaloInputs& in, double* phi, const SolveOpts&
   EAF_CUDA(cudaEventRecord(h->ev[3], h->st));
   EAF_CUDA(eaf::launch_unpack_f64(h->d, h->s.x, phi, h->st));
   EAF_CUDA(cudaEventRecord(h->ev[4], h->st));
-  h->last_kernels = 2 + kernels;  // pack, the solver's, unpack
+  h->last_kernels = 2 + ran.kernels;  // pack, the solver's, unpack
+  h->last_resident = ran.resident;
   return EAF_OK;
 }
 

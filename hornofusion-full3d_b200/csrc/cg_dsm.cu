@@ -1090,7 +1090,7 @@ cudaError_t launch_push_selftest(const GroupWs& ws, uint64_t timeout_ns, cudaStr
 
 cudaError_t launch_cg_f64_dsm(const MeshDims& d, const SysF64& s, const GroupWs& ws,
                               int max_iter, double tol, int block, int cluster,
-                              cudaStream_t st, int signal, uint64_t timeout_ns) {
+                              cudaStream_t st, int signal, uint64_t timeout_ns, int* ran) {
   if (cluster < 1 || cluster > kMaxClusterSize || block < 32 || block > 1024 ||
       block % 32 != 0 || d.n > dsm_max_cells(cluster))
     return cudaErrorInvalidValue;
@@ -1106,6 +1106,9 @@ cudaError_t launch_cg_f64_dsm(const MeshDims& d, const SysF64& s, const GroupWs&
   // The default signalling pushes where a thread's cells fit its registers.
   const int cells = signal == kDsmSignalMbarrier ? 0 : push_cells(d, a.chunk, block);
   a.reach = push_reach(d, a.chunk);
+  if (ran)
+    *ran = cells ? EAF_CG_RESIDENT_PUSHED
+           : signal == kDsmSignalMbarrier ? EAF_CG_RESIDENT_MBARRIER : EAF_CG_RESIDENT_BARRIER;
   const size_t smem = cells ? push_smem_bytes(a.reach, a.chunk, cells, block) : dsm_smem_bytes(a.chunk);
   const void* k = cells ? push_kernel(cells, block, cluster)
                   : signal == kDsmSignalMbarrier ? (const void*)cg_dsm_kernel<true>

@@ -146,12 +146,13 @@ int max_active_clusters(int block, long long n, int cluster);
 // `signal` picks how a block signals its partials: kDsmSignalDefault (pushed
 // with z where a thread's one or two cells fit its registers, else a full
 // cluster barrier) or kDsmSignalMbarrier (remote mbarrier arrivals).
+// `ran` (if not null) receives the form launched, EAF_CG_RESIDENT_*.
 constexpr int kDsmSignalDefault = 1;
 constexpr int kDsmSignalMbarrier = 2;
 cudaError_t launch_cg_f64_dsm(const MeshDims& d, const SysF64& s, const GroupWs& ws,
                               int max_iter, double tol, int block, int cluster,
                               cudaStream_t st, int signal = kDsmSignalDefault,
-                              uint64_t timeout_ns = 2000000000ull);
+                              uint64_t timeout_ns = 2000000000ull, int* ran = nullptr);
 int dsm_max_cells(int cluster);
 // Whether one cluster of `cluster` blocks of `block` threads holding an
 // n-cell system can be resident on the current device.
@@ -175,11 +176,15 @@ bool runs_resident(const SolverLaunch& L, long long n, bool allowed);
 // Enqueues the plain FP64 solver (reference form) on launch L: the flat,
 // cluster or cluster-resident kernel; `slot_doubles` is the size of ws.part.
 // `resident`: 0 never the cluster-resident kernel, 1 it with its default
-// signalling, 2 it with mbarrier signalling. `kernels`: how many were launched.
+// signalling, 2 it with mbarrier signalling. `ran` (if not null): what was launched.
+struct SolverRan {
+  int kernels;
+  int resident;  // EAF_CG_RESIDENT_*
+};
 cudaError_t launch_f64_solver(const SolverLaunch& L, int resident, const MeshDims& d,
                               const SysF64& s, const GroupWs& ws, size_t slot_doubles,
                               int max_iter, double tol, uint64_t timeout_ns, cudaStream_t st,
-                              int* kernels = nullptr);
+                              SolverRan* ran = nullptr);
 // Single-reduction (Chronopoulos-Gear) form of the same PCG: one group
 // all-reduce per iteration; uses s0/s1 and reuses r, z, q, p2 as the
 // double-buffered r and w = A M^-1 r.

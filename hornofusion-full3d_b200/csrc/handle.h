@@ -30,6 +30,7 @@ struct eaf_cg {
   int kernel;          // EAF_CG_KERNEL_*: per-thread loads or bulk-copy streaming
   int last_stream;     // the last FP64 solve's flat kernel: 0 loads, 1 stream, 2 slots, 3 keep
   double* trace_d;     // mixed form: per refinement step trace (lazy)
+  int last_resident;   // EAF_CG_RESIDENT_* of the last solve
   int trace_cap;       // refinement steps trace_d holds
   int sms;
   uint64_t timeout_ns;

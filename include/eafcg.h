@@ -160,6 +160,14 @@ int eaf_cg_last_cluster(eaf_cg_t h, int* cluster_blocks);
  * launch. No reference counterpart. */
 int eaf_cg_set_resident(eaf_cg_t h, int resident);
 
+/* Form of the cluster-resident kernel that the handle's last solve ran. No
+ * reference counterpart. */
+#define EAF_CG_RESIDENT_NONE 0    /* another kernel (eaf_cg_last_kernel, _last_cluster) */
+#define EAF_CG_RESIDENT_BARRIER 1
+#define EAF_CG_RESIDENT_MBARRIER 2
+#define EAF_CG_RESIDENT_PUSHED 3
+int eaf_cg_last_resident(eaf_cg_t h, int* form);
+
 /* Kernel of the plain FP64 solve on a flat (cluster-free) grid: per-thread
  * loads (EAF_CG_KERNEL_LOADS), or each phase's operands staged in shared
  * memory by bulk copies a few tiles ahead of use (EAF_CG_KERNEL_STREAM),
