@@ -71,6 +71,7 @@ struct SrvRun {
   double* stage[9];  // aW..Su inputs and phi (the device-resident warm start)
   double* h_phi;     // pinned download buffer for pageable phi_out
   bool busy;
+  bool fresh;        // phi is to be zeroed by the first batch, on its stream
 };
 
 struct SrvTicket {
@@ -290,7 +291,11 @@ bool launch(eaf_srv* s, std::unique_lock<std::mutex>& lk) {
                           sl->st);
   }
   for (int i = 0; i < nb && e == cudaSuccess; ++i) {
-    const SrvRun* r = pick[i].run;
+    SrvRun* r = pick[i].run;
+    // (the streams are non-blocking: nothing orders them behind a memset on the
+    // default stream)
+    if (r->fresh) e = cudaMemsetAsync(r->stage[8], 0, (size_t)r->nh * sizeof(double), sl->st);
+    if (e == cudaSuccess) r->fresh = false;
     for (int k = 0; k < 8 && e == cudaSuccess; ++k)
       e = cudaMemcpyAsync(r->stage[k], pick[i].in[k], (size_t)r->nh * sizeof(double),
                           cudaMemcpyHostToDevice, sl->st);
@@ -533,7 +538,7 @@ int eaf_srv_open_run(eaf_srv_t s, int nr, int nth, int nz, int* run_id) {
     }
     for (int k = 0; k < 9 && e == cudaSuccess; ++k)
       e = cudaMalloc((void**)&r->stage[k], (size_t)nh * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemset(r->stage[8], 0, (size_t)nh * sizeof(double));
+    r->fresh = true;
     if (e == cudaSuccess) e = cudaHostAlloc((void**)&r->h_phi, (size_t)nh * sizeof(double), 0);
   }
   std::lock_guard<std::mutex> lk(s->m);

@@ -10,10 +10,12 @@ import pytest
 from conftest import ROOT, gen, pkg
 
 
-def test_no_copy_on_the_default_stream():
-    with open(os.path.join(ROOT, "hornofusion-full3d_b200", "csrc", "batch.cu")) as f:
+# (the server's streams are non-blocking too)
+@pytest.mark.parametrize("unit", ["batch.cu", "serve.cu"])
+def test_no_copy_on_the_default_stream(unit):
+    with open(os.path.join(ROOT, "hornofusion-full3d_b200", "csrc", unit)) as f:
         code = re.sub(r"//[^\n]*", "", f.read())
-    assert "b->st" in code
+    assert "cudaStreamNonBlocking" in code
     assert re.findall(r"\bcuda(?:Memcpy|Memset)\s*\(", code) == []
 
 
