@@ -448,7 +448,7 @@ static_assert(offsetof(PushSmem, rz) == 8 * kMaxClusterSize &&
 // What a block's all-reduces need, set up once (shared-memory addresses).
 struct Pusher {
   int rank;
-  uint32_t phases;             // parity of the phase that is not complete yet, bit per barrier
+  uint32_t phases;             // completion parity expected next, bit per barrier
   uint32_t smem, bar;          // this block's PushSmem and barriers
   uint32_t to_smem, to_bar;    // those of lane's target block (lane & 15)
   uint32_t z_bytes;            // bytes of z a block receives per exchange
@@ -562,10 +562,14 @@ constexpr uint32_t kAtPq = 0, kAtRz = 8 * kMaxClusterSize, kAtPre = 24 * kMaxClu
 // waits for the partials of the (at most) CMAX blocks, whose slots beyond the
 // cluster's size hold zeros, and folds them in rank order. Two values are
 // pushed by the two halves of warp 0. The barrier's next phase, which will
-// carry `next` bytes, is opened on the way out. False if the wait gave up (the
-// phase then stays open: an arrival on it would be one too many); a block leaves
-// as one.
-template <int NV, int KIND, int CMAX>
+// carry `next` bytes, is opened by a thread that has seen this one complete (the
+// others still find it so: nothing pushes into the next before this block's
+// threads have met). False if the wait gave up; that thread then leaves the open
+// phase alone, which an arrival more would corrupt. A block leaves as one: before
+// the fold (EARLY) or behind it, whichever the registers bear better (50
+// iterations: two cells a thread, 18x36x24, 157.6 us before, 159.8 behind; one cell,
+// 10x20x12, 92.2 before, 90.1 behind).
+template <int NV, int KIND, int CMAX, bool EARLY = false>
 __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t next, Pusher& x) {
   constexpr int kPairs = (NV + 1) / 2;  // values go two by two
   constexpr int kTwo = NV >= 2 ? 2 : 1;
@@ -607,6 +611,7 @@ __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t nex
   }
   const uint32_t bar = x.bar + 8u * KIND;
   const uint32_t want = (x.phases >> KIND) & 1u;
+  x.phases ^= 1u << KIND;
   bool ok = true;
   if (!mbar_test_cluster(bar, want)) {
     const uint64_t t0 = global_ns();
@@ -622,10 +627,9 @@ __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t nex
       }
     }
   }
+  if (threadIdx.x == blockDim.x - 1 && ok) push_expect(bar, next);
   ok = __syncthreads_and(ok) != 0;
-  if (!ok) return false;
-  x.phases ^= 1u << KIND;
-  if (threadIdx.x == blockDim.x - 1) push_expect(bar, next);
+  if (EARLY && !ok) return false;
   const uint32_t part = x.smem + kAt;
   if (NV == 1) {
     double t[CMAX];
@@ -656,7 +660,7 @@ __device__ __forceinline__ bool push_allsum(double (&v)[NV], int C, uint32_t nex
       v[m] = t;
     }
   }
-  return true;
+  return ok;
 }
 
 // The end of a solve, every thread of the cluster: no block leaves while another
@@ -675,9 +679,12 @@ __device__ __forceinline__ void push_leave(PushSmem& ps, const Pusher& x, int C,
   cluster_sync_all();
   if (*(volatile int*)&ps.gave_up == 0) return;
   const uint64_t t0 = global_ns();
-  for (int b = 0; b < 2; ++b)
-    for (int n = 0; n < 4096 && !mbar_test_cluster(x.bar + 8u * b, (x.phases >> b) & 1u); ++n)
+  for (int b = 0; b < 2; ++b) {
+    // (of the two parities, the open phase's is the one that has not completed)
+    const uint32_t bar = x.bar + 8u * b, open = mbar_test_cluster(bar, 0u) ? 1u : 0u;
+    for (int n = 0; n < 4096 && !mbar_test_cluster(bar, open); ++n)
       if (global_ns() - t0 > kPushDrainNs) break;
+  }
   __syncthreads();
   cluster_sync_all();
 }
@@ -824,7 +831,7 @@ __device__ void push_body(const DsmArgs& a, double* sm, PushSmem& ps, int C, int
     v3[1] = v3[1] + r[m] * r[m];
     v3[2] = v3[2] + r[m] * z[m];
   }
-  bool ok = push_allsum<3, 1, CMAX>(v3, C, rz_bytes, px);
+  bool ok = push_allsum<3, 1, CMAX, R == 2>(v3, C, rz_bytes, px);
   const double bnorm = sqrt(v3[0]);
   double residual = 0.0, rr = 0.0;
   int n_iter = 0;
@@ -876,7 +883,7 @@ __device__ void push_body(const DsmArgs& a, double* sm, PushSmem& ps, int C, int
         q[m] = y;
         v1[0] = v1[0] + p[m] * y;
       }
-      if (!(ok = push_allsum<1, 0, CMAX>(v1, C, pq_bytes, px))) break;
+      if (!(ok = push_allsum<1, 0, CMAX, R == 2>(v1, C, pq_bytes, px))) break;
       const double pq = v1[0];
       if (fabs(pq) < kSmall) break;
       const double alpha = rz / pq;
@@ -895,7 +902,7 @@ __device__ void push_body(const DsmArgs& a, double* sm, PushSmem& ps, int C, int
         v2[0] = v2[0] + r[m] * r[m];
         v2[1] = v2[1] + r[m] * z[m];
       }
-      if (!(ok = push_allsum<2, 1, CMAX>(v2, C, rz_bytes, px))) break;
+      if (!(ok = push_allsum<2, 1, CMAX, R == 2>(v2, C, rz_bytes, px))) break;
       rr = v2[0];
       n_iter = iter;
       if (!(rr > surely_above)) {
