@@ -161,6 +161,10 @@ SolverLaunch choose_launch(int nr, int nth, int nz, int sms, int req_block, int 
       // 6.5 / 8.4, 121,296 6.9 / 8.3, 193,971 7.9 / 8.4, 389,376 10.3 / 10.9,
       // 878,560 15.0 / 16.9; blocks of 256 or 1024 threads were slower from
       // 120,000 cells on and within 2 % below.
+      // (A lone solve's times. Several handles' solves share the SMs up to one cell
+      // a thread, cg_keep_kernel_ptr; beyond, they follow each other, where the
+      // smaller grids ran side by side: 78,540 cells, 50 iterations, us a solve by
+      // 1, 2, 4 threads, 474 / 245 / 142 then, 377 / 345 / 343 now.)
       // Well beyond L2 the prefetching 1024-thread kernel takes over: 1,212,960
       // cells 25.5 (512) / 26.5 (1024), 1,408,000 33.5 / 30.2, 2,800,000 74.0 / 59.7.
       g = sms < 32 * kPerLane ? sms : 32 * kPerLane;

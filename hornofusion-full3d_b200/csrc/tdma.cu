@@ -36,7 +36,9 @@
 // exact, every value is the sequential recurrence's, whatever the scan
 // delivered. Two passes are the rule, because a segment contracts an error of
 // a few ulps below a rounding; a line without contraction takes up to 32,
-// about the sequential cost. A pass costs 42 cycles an element (five
+// about the sequential cost. (60x120x84, two sweeps, ms, a lane a line 8.5 on
+// all: random links 1.62, conduction on the cylinder with a sink of 1e-2 of the
+// links 1.84, of 1e-6 2.05, links of one direction 1e6 times the others' 3.29.) A pass costs 42 cycles an element (five
 // dependent FP64 operations) plus a shuffle, so the passes needed times K is
 // what counts: K = 4 on as few lanes as the line fills, more only beyond 128
 // elements (one element a lane needs four to five passes and five scan steps).
@@ -1073,8 +1075,13 @@ __global__ void div_check_kernel(long long n, unsigned long long seed,
   atomicAdd(counts + 1, fast);
 }
 
-// Elements per lane of a line of L: four (see the file comment), beyond 128
-// the next instantiated size.
+// Elements per lane of a line of L: four (see the file comment), beyond 128 the
+// next instantiated size. A lane pays for K elements whether the line fills them
+// or not, and the sizes between the powers of two save a part of that (two sweeps,
+// ms, with / without them: z lines of 160 1.76 / 1.96, 300 2.75 / 3.19, 700 4.20 /
+// 4.71). From 16 on the 255 registers do not hold a lane's arrays (K = 32 spills
+// 3.7 KB), and still no length is slower than a lane a line was: 200 10.2 -> 2.1,
+// 300 15.0 -> 2.75, theta lines of 512 7.1 -> 2.6, of 1024 13.9 -> 5.2.
 int line_k(int L) {
   const int k = (L + 31) / 32;
   return k <= 4 ? 4 : k <= 6 ? 6 : k <= 8 ? 8 : k <= 12 ? 12 : k <= 16 ? 16 : k <= 24 ? 24 : 32;
