@@ -17,6 +17,29 @@ def grown(call):
     return before - torch.cuda.mem_get_info()[0]
 
 
+def load_sweep_kernels():
+    """Sweeps of a small mesh first: a kernel's first launch may take memory too."""
+    g = gen()
+    s = g.make_transport_system(12, 24, 16, seed=4)
+    with pkg().CGSolver(12, 24, 16) as cg:
+        cg.tdma(s.arrays(), g.zeros_phi(12, 24, 16), 2)
+
+
+def fill_device(leave):
+    """Tensors that take the device's free memory but about `leave` bytes."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held, step = [], 1 << 60
+    while torch.cuda.mem_get_info()[0] > leave + (16 << 20) and step > (1 << 20):
+        step = min(step, torch.cuda.mem_get_info()[0] - leave)
+        try:
+            held.append(torch.empty(step, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            step //= 2
+    return held
+
+
 def on_device(f):
     import torch
     dev = f.copy()
@@ -45,6 +68,7 @@ def test_transport_scratch():
     s = g.make_transport_system(*dims, seed=1)
     dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in s.arrays()]
     phi = torch.zeros(g.halo_shape(*dims), dtype=torch.float64, device="cuda")
+    load_sweep_kernels()
     with eaf.CGSolver(*dims) as cg:
         for _ in range(2):
             assert grown(lambda: cg.tdma(dev, phi, 1, device_ptrs=True)) == 0
@@ -87,19 +111,16 @@ def test_records_built_again_without_room():
     dims = (60, 120, 84)
     s = g.make_transport_system(*dims, seed=4)
     phi0 = np.random.default_rng(2).normal(size=g.halo_shape(*dims))
-    small = g.make_transport_system(12, 24, 16, seed=4)
-    sweeps((12, 24, 16), g.zeros_phi(12, 24, 16), (2,), small)  # (the kernels are loaded)
+    load_sweep_kernels()
 
     dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in s.arrays()]
     a, b = torch.from_numpy(phi0.copy()).cuda(), phi0.copy()
     with eaf.CGSolver(*dims) as cg:
-        torch.cuda.synchronize()
-        torch.cuda.empty_cache()
-        fill = torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8,
-                           device="cuda")
+        held = fill_device(64 << 20)
+        assert torch.cuda.mem_get_info()[0] < 90 << 20  # (the records need 94 MB)
         cg.tdma(dev, a, 3, device_ptrs=True)
         assert cg.last_timing()["kernels"] == 27
-        del fill
+        del held
         torch.cuda.empty_cache()
         cg.tdma(dev, a, 2, device_ptrs=True)
         assert cg.last_timing()["kernels"] == 15
